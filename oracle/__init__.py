@@ -358,7 +358,7 @@ def build_reference(ref_root=None, jobs=8):
     ref_root: the reference's source tree; QMIV_REFERENCE_ROOT is read when it is not given. Without
     either, nothing is built."""
     ref_root = ref_root or os.environ.get("QMIV_REFERENCE_ROOT")
-    if not ref_root or not os.path.isdir(ref_root):
+    if not ref_root or not os.path.exists(os.path.join(ref_root, "apps", "QMIV", "src", "main_QMIV.cpp")):
         return False
     subprocess.run(["make", "-s", "-C", HERE, f"-j{jobs}", "ref", f"REF={ref_root}"], check=True)
     if os.path.exists(os.path.join(os.path.dirname(HERE), "qmiv_b200", "libqmiv_b200.so")):
