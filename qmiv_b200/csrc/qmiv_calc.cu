@@ -147,7 +147,7 @@ qmiv_status PairPipeline::configure(qmiv_ctx_s* ctx, const Shape& shape, const q
 {
   ctx_ = ctx; shape_ = shape; prm_ = prm; R_ = search_range;
   for(int c = 0; c < 4; c++) { maxdiff_[c] = round_f32_half_away(prm.unc[c] * (float)shape.maxv); }  // xGlobClrDiff.cpp:76
-  fp32_ok_ = cps_fp32_exact(shape.maxv, prm.cws, maxdiff_);
+  fp32_ok_ = cps_key_exact(search_range, shape.sx, shape.sy, shape.maxv, prm.cws, maxdiff_);
   ns_ = num_scales(shape.W, shape.H);
   int32_t w = shape.W, h = shape.H;
   for(int s = 0; s < 5; s++)
@@ -342,7 +342,7 @@ qmiv_status PairPipeline::enqueue_t(const Img& in0, const Img& in1, uint32_t mas
     int32_t mag[4];
     for(int c = 0; c < 4; c++) { ra.gcd_override[c] = gcd_override_[c]; mag[c] = gcd_override_[c] < 0 ? -gcd_override_[c] : gcd_override_[c]; }
     ra.gcd_override_on = 1;
-    ra.fp32_ok = cps_fp32_exact(S.maxv, prm_.cws, mag);
+    ra.fp32_ok = cps_key_exact(R_, S.sx, S.sy, S.maxv, prm_.cws, mag);
   }
   ra.row_sd = pa.row_sd; ra.row_ssd = pa.row_ssd; ra.out = dout;
   { const int t = prof_begin(s); QMIV_CUDA(launch_reduce(ra, s)); prof_end(s, QMIV_STAGE_REDUCE, t); }
@@ -353,6 +353,7 @@ qmiv_status PairPipeline::enqueue_t(const Img& in0, const Img& in1, uint32_t mas
     CpsArgs ca{};
     ca.in0 = in0; ca.in1 = in1; ca.W = S.W; ca.H = S.H; ca.maxv = S.maxv; ca.clip = clip;
     for(int c = 0; c < 3; c++) { ca.wi[c] = prm_.cws[c]; ca.wf[c] = (float)prm_.cws[c]; }
+    for(int c = 0; c < 3; c++) { ca.gmax[c] = gcd_override_on_ ? gcd_override_[c] : maxdiff_[c]; }
     ca.gcd_src = dout; ca.rows = cps_rows_.as<uint32_t>();
     ca.scp0 = need_scp ? const_cast<void*>(scp(0)) : nullptr;
     ca.scp1 = need_scp ? const_cast<void*>(scp(1)) : nullptr;

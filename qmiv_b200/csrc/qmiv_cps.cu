@@ -1,5 +1,6 @@
-// Corresponding-pixel-shift search (libs/pmbb-ivqm/src/xCorrespPixelShiftSSE.cpp:18-127) for
-// sm_100a: persistent CTAs, TMA tile loads, 4 x 2 pixels per thread in the search.
+// Corresponding-pixel-shift search (libs/pmbb-ivqm/src/xCorrespPixelShiftSSE.cpp:18-127) of 4:2:2 and
+// 4:4:4 pictures for sm_100a: persistent CTAs, TMA tile loads, 4 x 2 pixels per thread in the search.
+// (4:2:0: qmiv_cps420.cu.)
 //
 // Per tile of 128 x TH output pixels (TH = 32, or 16 when shared memory is short or the autotuner
 // prefers two CTAs per SM) a CTA of 2 x TH / 4 warps
@@ -8,9 +9,8 @@
 //      are issued as soon as tile n's raw samples are converted, so they land during its search;
 //   2. converts them into two float4 tiles (Y, Cb, Cr, q + 2^23), q = sum_c w_c * ref_c^2,
 //      reading every sample at its clamped picture coordinate (the reference's edge-replicated
-//      margin, apps/QMIV/src/xAppQMIV.cpp:353 and :899) and the chroma of 4:2:0 / 4:2:2 at
-//      (x >> sx, y >> sy) (the nearest upsampling of libs/pmbb-core/src/xPixelOpsSTD.cpp:30-87);
-//      4:2:0 tiles at an even search range are converted as 2x2 units sharing one chroma sample;
+//      margin, apps/QMIV/src/xAppQMIV.cpp:353 and :899) and the chroma of 4:2:2 at (x >> 1, y) (the
+//      nearest upsampling of libs/pmbb-core/src/xPixelOpsSTD.cpp:30-87);
 //   3. searches both directions. A thread owns 4 rows x 2 columns of output pixels, so each
 //      staged reference pixel is loaded once per thread for up to 8 of its pixels; the winners'
 //      candidate codes go to shared memory;
@@ -34,16 +34,9 @@
 // y * RP + (x & 1) * Q + (x >> 1). A warp reading column 2 * lane + rx for fixed rx touches 32
 // consecutive float4 (no bank conflict), and with Q = 4 (mod 8) the conversion's stores of 32
 // consecutive columns are conflict-free as well.
-#include "qmiv_kernels.cuh"
+#include "qmiv_cps.cuh"
 
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
-#include <algorithm>
-#include <atomic>
 #include <cstring>
-#include <map>
-#include <mutex>
 
 namespace qmiv {
 
@@ -55,7 +48,6 @@ constexpr uint32_t kKeyBase  = 0x49800000u;  // bit pattern of 2^20f
 __constant__ uint32_t c_key_scale = 128u;
 constexpr uint32_t kBiasBits = 0x4B000000u;  // bit pattern of 2^23f
 constexpr unsigned kFull     = 0xffffffffu;
-constexpr long long kWaitCycles = 1LL << 31; // bound of one tile-load wait (about a second)
 
 template <int R, int WY>
 struct Geo
@@ -70,41 +62,6 @@ struct Geo
   static constexpr uint32_t kTileBytes = (uint32_t)SH * RP * 16u;
   static constexpr uint32_t kCodeBytes = 2u * TH * TW; // winners' candidate codes [dir][TH][TW]
 };
-
-struct CpsGeomArgs
-{
-  int32_t  ntx, ntiles;
-  int32_t  use_tma;
-  int32_t  ax;                 // 16 bytes in samples: TMA boxes start this far left of the tile
-  int32_t  bwl, bhl, bwc, bhc; // raw box sizes in samples (luma, chroma)
-  int32_t  sx, sy;             // chroma subsampling shifts
-  uint32_t off[2][3];          // byte offsets of the raw boxes in shared memory
-  uint32_t raw_bytes;          // raw region, multiple of 128
-  uint32_t tx_bytes;           // bytes the six copies of one tile deliver
-  int32_t* status;             // PairOut::flags: bit 3 = a tile load did not complete
-};
-
-struct alignas(64) CpsKernelArgs
-{
-  CUtensorMap map[2][3];       // [picture][plane]
-  CpsArgs     a;
-  CpsGeomArgs g;
-};
-
-// ---- TMA / mbarrier ---------------------------------------------------------------------------
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar)
-{
-  asm volatile(
-    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-    ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-
-// ---- tile loads ---------------------------------------------------------------------------------
-// Tensor maps written to global memory by a host copy are made visible to the TMA unit
-__device__ __forceinline__ void fence_tensormap_acquire(const CUtensorMap* map)
-{
-  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
-}
 
 template <int R, int WY, bool GMAPS>
 __device__ __forceinline__ void issue_tile(const CpsKernelArgs& k, unsigned char* raw, uint64_t* bar, int t)
@@ -208,86 +165,6 @@ __device__ void convert(const CpsArgs& a, const CpsGeomArgs& g, const unsigned c
         frow[16 * kk] = make_float4(y, u, v, fmaf(w2, v * v, fmaf(w1, u * u, fmaf(w0, y * y, kBias))));
       }
     }
-  }
-}
-
-// Two neighbouring samples of a raw row, as one 32-bit word (2-byte samples) or the low half of one
-// (1-byte samples); the address is even in samples.
-template <typename T>
-__device__ __forceinline__ uint32_t load_pair(const T* p)
-{
-  if constexpr(sizeof(T) == 2) { return *reinterpret_cast<const uint32_t*>(p); }
-  else { return *reinterpret_cast<const uint16_t*>(p); }
-}
-// Byte selectors placing the first / second sample of a pair into the low bits of 0x4B000000
-// (2^23), whose float value minus 2^23 is then the sample itself.
-template <typename T> struct PairSel;
-template <> struct PairSel<uint16_t> { static constexpr uint32_t lo = 0x7410u, hi = 0x7432u; };
-template <> struct PairSel<uint8_t>  { static constexpr uint32_t lo = 0x7440u, hi = 0x7441u; };
-__device__ __forceinline__ float pair_f(uint32_t pr, uint32_t sel) { return __uint_as_float(__byte_perm(pr, kBiasBits, sel)) - kBias; }
-
-// raw boxes -> float4 tiles for 4:2:0 pictures and an even search range. The staged samples then
-// start at even picture coordinates and fall into 2x2 units that share one chroma sample; a thread
-// converts whole units: each unit row's two luma samples from one load, the chroma pair and the
-// chroma part of q (w1 Cb^2 + w2 Cr^2 + 2^23) once. Coordinates are clamped as in `convert`: a unit
-// lies either wholly inside or wholly outside the picture in each direction (even W and H), and the
-// clamped column pair and the selectors reproduce the edge replication; tiles whose halo lies inside
-// the picture (INTERIOR) skip the clamps. The float4 values are those of `convert`: every term is an
-// integer below 2^24, so the changed order of the sums is exact.
-template <typename T, int R, int WY, bool INTERIOR>
-__device__ void convert420(const CpsArgs& a, const CpsGeomArgs& g, const unsigned char* raw, float4* F0, float4* F1,
-                           int x0, int y0)
-{
-  using G = Geo<R, WY>;
-  static_assert(R % 2 == 0, "units start at even coordinates");
-  constexpr int UC = G::SW / 2, UR = G::SH / 2, NU = UC * UR;
-  const int W = a.W, H = a.H;
-  const int cw = W >> 1, chh = H >> 1;
-  const int ax = g.ax, bwl = g.bwl, bwc = g.bwc;
-  const int xl = x0 - ax, yl = y0 - R, xc = (x0 >> 1) - ax, yc = (y0 - R) >> 1;
-  const float w0 = a.wf[0], w1 = a.wf[1], w2 = a.wf[2];
-  // the geometry is read once: the tile stores below could alias the shared argument copy
-  const uint32_t offl[2] = { g.off[0][0], g.off[1][0] }, offu[2] = { g.off[0][1], g.off[1][1] },
-                 offv[2] = { g.off[0][2], g.off[1][2] };
-  #pragma unroll 1
-  for(int u = threadIdx.x; u < 2 * NU; u += G::NT)
-  {
-    const int f = u >= NU ? 1 : 0;
-    const int r = u - f * NU;
-    const int ur = r / UC, uc = r - ur * UC;
-    const T* rl = reinterpret_cast<const T*>(raw + (f ? offl[1] : offl[0]));
-    const T* ru = reinterpret_cast<const T*>(raw + (f ? offu[1] : offu[0]));
-    const T* rv = reinterpret_cast<const T*>(raw + (f ? offv[1] : offv[0]));
-    uint32_t l0, l1, s0 = PairSel<T>::lo, s1 = PairSel<T>::hi;
-    int co;
-    if(INTERIOR)
-    {
-      // the tile and its halo lie inside the picture: unit (ur, uc) is raw luma (2 ur, ax - R + 2 uc)
-      // and raw chroma (ur, ax - R / 2 + uc)
-      const T* p = rl + 2 * ur * bwl + (ax - R) + 2 * uc;
-      l0 = load_pair<T>(p);
-      l1 = load_pair<T>(p + bwl);
-      co = ur * bwc + (ax - R / 2) + uc;
-    }
-    else
-    {
-      const int gx = x0 - R + 2 * uc, gy = y0 - R + 2 * ur;
-      const int px = clampi(gx, 0, W - 2);
-      s0 = gx < W ? PairSel<T>::lo : PairSel<T>::hi;
-      s1 = gx >= 0 ? PairSel<T>::hi : PairSel<T>::lo;
-      const int gy0 = clampi(gy, 0, H - 1), gy1 = clampi(gy + 1, 0, H - 1);
-      l0 = load_pair<T>(rl + (gy0 - yl) * bwl + (px - xl));
-      l1 = load_pair<T>(rl + (gy1 - yl) * bwl + (px - xl));
-      co = (clampi(gy >> 1, 0, chh - 1) - yc) * bwc + clampi(gx >> 1, 0, cw - 1) - xc;
-    }
-    const float cu = u2f_exact(ru[co]), cv = u2f_exact(rv[co]);
-    const float qc = fmaf(w2, cv * cv, fmaf(w1, cu * cu, kBias));
-    const float y00 = pair_f(l0, s0), y01 = pair_f(l0, s1), y10 = pair_f(l1, s0), y11 = pair_f(l1, s1);
-    float4* d = (f ? F1 : F0) + 2 * ur * G::RP + uc;
-    d[0]             = make_float4(y00, cu, cv, fmaf(w0, y00 * y00, qc));
-    d[G::Q]          = make_float4(y01, cu, cv, fmaf(w0, y01 * y01, qc));
-    d[G::RP]         = make_float4(y10, cu, cv, fmaf(w0, y10 * y10, qc));
-    d[G::RP + G::Q]  = make_float4(y11, cu, cv, fmaf(w0, y11 * y11, qc));
   }
 }
 
@@ -758,19 +635,7 @@ __device__ __forceinline__ void cps_loop(int ntiles, const Locate& locate, uint3
       __syncthreads();
     }
     if(a.clip < (sizeof(T) == 1 ? 0xffu : 0xffffu)) { convert<T, R, WY, true>(a, g, raw, F0, F1, x0, y0); }
-    else
-    {
-      if constexpr(R % 2 == 0)
-      {
-        if(g.sx == 1 && g.sy == 1)
-        {
-          if(x0 >= R && y0 >= R && x0 + G::TW + R <= a.W && y0 + G::TH + R <= a.H) { convert420<T, R, WY, true>(a, g, raw, F0, F1, x0, y0); }
-          else { convert420<T, R, WY, false>(a, g, raw, F0, F1, x0, y0); }
-        }
-        else { convert<T, R, WY, false>(a, g, raw, F0, F1, x0, y0); }
-      }
-      else { convert<T, R, WY, false>(a, g, raw, F0, F1, x0, y0); }
-    }
+    else { convert<T, R, WY, false>(a, g, raw, F0, F1, x0, y0); }
     __syncthreads();
     // the raw boxes are free again: the next tile's copies overlap this tile's search
     const int tn = t + (int)gridDim.x;
@@ -838,61 +703,7 @@ __global__ void __launch_bounds__(64 * WY, WY == 4 ? 2 : 1) k_cps_multi(const Cp
 }
 
 // ---- host -------------------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn()
-{
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-       q == cudaDriverEntryPointSuccess)
-    {
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }
-  });
-  return fn;
-}
-
-// One 2D tensor map per plane. Returns false when TMA cannot take the plane (alignment, pitch).
-bool encode_plane(CUtensorMap* m, const void* p, int32_t w, int32_t h, int64_t pitch_elems, int esz, int bw, int bh)
-{
-  const uint64_t pitch = (uint64_t)pitch_elems * (uint64_t)esz;
-  if(((uintptr_t)p & 15) != 0 || (pitch & 15) != 0 || pitch >= (1ULL << 40) || w <= 0 || h <= 0) { return false; }
-  PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
-  if(fn == nullptr) { return false; }
-  const cuuint64_t dims[2] = { (cuuint64_t)w, (cuuint64_t)h };
-  const cuuint64_t strides[1] = { (cuuint64_t)pitch };
-  const cuuint32_t box[2] = { (cuuint32_t)bw, (cuuint32_t)bh };
-  const cuuint32_t estr[2] = { 1, 1 };
-  const CUresult r = fn(m, esz == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(p),
-                        dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
-}
-
-struct DevInfo
-{
-  int sms = 0, smem_optin = 0;
-};
-DevInfo dev_info(int dev)
-{
-  static std::mutex mu;
-  static DevInfo cache[64];
-  std::lock_guard<std::mutex> lk(mu);
-  if(dev < 0 || dev >= 64) { return DevInfo{ 1, 48 * 1024 }; }
-  if(cache[dev].sms == 0)
-  {
-    cudaDeviceGetAttribute(&cache[dev].sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&cache[dev].smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if(cache[dev].sms <= 0) { cache[dev].sms = 1; }
-  }
-  return cache[dev];
-}
-
-constexpr int kAlign = 128;
 constexpr size_t kStaticSmem = 1024;   // the kernel's static shared memory (argument copy), rounded up
-inline uint32_t align_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 
 // Geometry for one (R, WY, sample size, subsampling); returns the dynamic shared memory size.
 template <int R, int WY>
@@ -958,38 +769,11 @@ bool encode_maps(CpsKernelArgs& k, int esz)
   for(int f = 0; f < 2; f++)
   {
     const Img& im = f ? k.a.in1 : k.a.in0;
-    if(!encode_plane(&k.map[f][0], im.p[0], k.a.W, k.a.H, im.pitch[0], esz, k.g.bwl, k.g.bhl)) { return false; }
-    if(!encode_plane(&k.map[f][1], im.p[1], cw, ch, im.pitch[1], esz, k.g.bwc, k.g.bhc)) { return false; }
-    if(!encode_plane(&k.map[f][2], im.p[2], cw, ch, im.pitch[2], esz, k.g.bwc, k.g.bhc)) { return false; }
+    if(!cps_encode_plane(&k.map[f][0], im.p[0], k.a.W, k.a.H, im.pitch[0], esz, k.g.bwl, k.g.bhl)) { return false; }
+    if(!cps_encode_plane(&k.map[f][1], im.p[1], cw, ch, im.pitch[1], esz, k.g.bwc, k.g.bhc)) { return false; }
+    if(!cps_encode_plane(&k.map[f][2], im.p[2], cw, ch, im.pitch[2], esz, k.g.bwc, k.g.bhc)) { return false; }
   }
   return true;
-}
-
-// Raises the kernel's dynamic shared memory limit once per (kernel, device). The opt-in limit
-// covers the kernel's static shared memory (the argument copy) and the dynamic part together.
-template <typename F>
-cudaError_t configure_once(F* fn, int dev)
-{
-  static std::mutex mu;
-  static std::map<const void*, uint64_t> done;
-  const uint64_t bit = 1ULL << (dev & 63);
-  std::lock_guard<std::mutex> lk(mu);
-  uint64_t& m = done[reinterpret_cast<const void*>(fn)];
-  if(m & bit) { return cudaSuccess; }
-  cudaFuncAttributes fa{};
-  cudaError_t e = cudaFuncGetAttributes(&fa, fn);
-  if(e != cudaSuccess) { return e; }
-  e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_info(dev).smem_optin - (int)fa.sharedSizeBytes);
-  if(e == cudaSuccess) { m |= bit; }
-  return e;
-}
-
-template <typename F>
-int grid_for(F* fn, int threads, size_t smem, int ntiles, int dev)
-{
-  int occ = 1;
-  if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, threads, smem) != cudaSuccess || occ < 1) { occ = 1; }
-  return std::max(1, std::min(ntiles, dev_info(dev).sms * occ));
 }
 
 template <int R, int WY, typename T>
@@ -1054,6 +838,7 @@ cudaError_t launch_multi_r(const CpsKernelArgs* d, const int32_t* prefix, int np
 // (128 x 16 tiles) otherwise.
 int cps_pick_wy(int R, int esz, int sx, int sy)
 {
+  if(sx == 1 && sy == 1) { return cps420_fits(R, esz) ? kCpsForm420 : 0; }
   if(R <= 4 && cps_tile_fits(R, 8, esz, sx, sy)) { return 8; }
   if(cps_tile_fits(R, 4, esz, sx, sy)) { return 4; }
   return 0;
@@ -1061,6 +846,7 @@ int cps_pick_wy(int R, int esz, int sx, int sy)
 
 bool cps_tile_fits(int R, int wy, int esz, int sx, int sy)
 {
+  if(sx == 1 && sy == 1) { return false; }   // the 4:2:0 form has one tile shape
   int dev = 0;
   if(cudaGetDevice(&dev) != cudaSuccess) { return false; }
   CpsGeomArgs g{};
@@ -1076,6 +862,7 @@ cudaError_t cps_describe(void* desc, const CpsArgs& a, int R, int esz, int wy, C
   std::memset(&k, 0, sizeof(k));
   k.a = a;
   k.g.status = const_cast<int32_t*>(&a.gcd_src->flags);
+  if(wy == kCpsForm420) { return cps420_describe(k, R, esz, plan); }
   size_t smem = 0;
   if(!plan_any(R, wy, k.g, smem, esz, a.in0.sx[1], a.in0.sy[1], a.W, a.H)) { return cudaErrorInvalidConfiguration; }
   k.g.use_tma = encode_maps(k, esz) ? 1 : 0;
@@ -1093,6 +880,7 @@ cudaError_t launch_cps_multi(const void* d_descs, const int32_t* d_prefix, int n
   cudaError_t e = cudaGetDevice(&dev);
   if(e != cudaSuccess) { return e; }
   const CpsKernelArgs* d = static_cast<const CpsKernelArgs*>(d_descs);
+  if(wy == kCpsForm420) { return cps420_launch_multi(d, d_prefix, npairs, ntiles, R, esz, s); }
   auto go = [&](auto tag) -> cudaError_t {
     using T = decltype(tag);
     switch(R)
@@ -1132,6 +920,11 @@ bool cps_fp32_exact(int32_t maxv, const int32_t w[3], const int32_t maxdiff[3])
   return true;
 }
 
+bool cps_key_exact(int R, int sx, int sy, int32_t maxv, const int32_t w[3], const int32_t maxdiff[3])
+{
+  return sx == 1 && sy == 1 ? cps_shared_key(R, maxv, w, maxdiff, nullptr, nullptr) : cps_fp32_exact(maxv, w, maxdiff);
+}
+
 template <typename T>
 cudaError_t launch_cps(const CpsArgs& a, int R, cudaStream_t s)
 {
@@ -1139,6 +932,11 @@ cudaError_t launch_cps(const CpsArgs& a, int R, cudaStream_t s)
   std::memset(&k, 0, sizeof(k));
   k.a = a;
   k.g.status = const_cast<int32_t*>(&a.gcd_src->flags);
+  if(a.in0.sx[1] == 1 && a.in0.sy[1] == 1)
+  {
+    const cudaError_t e = cps420_describe(k, R, (int)sizeof(T), nullptr);
+    return e != cudaSuccess ? e : cps420_launch(k, R, (int)sizeof(T), s);
+  }
   switch(R)
   {
   case 1: return launch_r<1, T>(k, s);

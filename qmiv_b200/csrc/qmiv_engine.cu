@@ -68,7 +68,7 @@ qmiv_status Engine::kind_for(const qmiv_pair_desc& d, PairKind*& out)
   QMIV_TRY(validate_params(k->prm));
   k->R = d.search_range;
   for(int c = 0; c < 4; c++) { k->maxdiff[c] = round_f32_half_away(prm_.unc[c] * (float)k->S.maxv); }  // xGlobClrDiff.cpp:76
-  k->fp32_ok = cps_fp32_exact(k->S.maxv, prm_.cws, k->maxdiff);
+  k->fp32_ok = cps_key_exact(k->R, k->S.sx, k->S.sy, k->S.maxv, prm_.cws, k->maxdiff);
   k->ns = num_scales(k->S.W, k->S.H);
   int32_t w = k->S.W, h = k->S.H;
   for(int s = 0; s < 5; s++)
@@ -693,7 +693,7 @@ void Engine::fill_tables(int n, const std::vector<PairKind*>& kind, const std::v
         const PairSlot& p = slots_[i];
         CpsArgs ca{};
         ca.in0 = in0[i]; ca.in1 = in1[i]; ca.W = K.S.W; ca.H = K.S.H; ca.maxv = K.S.maxv; ca.clip = clip_of(K);
-        for(int c = 0; c < 3; c++) { ca.wi[c] = prm_.cws[c]; ca.wf[c] = (float)prm_.cws[c]; }
+        for(int c = 0; c < 3; c++) { ca.wi[c] = prm_.cws[c]; ca.wf[c] = (float)prm_.cws[c]; ca.gmax[c] = K.maxdiff[c]; }
         ca.gcd_src = reinterpret_cast<PairOut*>(dbase + p.out);
         ca.rows = reinterpret_cast<uint32_t*>(dbase + p.cps_rows);
         if(p.need_scp)
@@ -930,7 +930,7 @@ bool Engine::tuning(int32_t W, int32_t H, int32_t bd, int32_t R, int32_t* tile_w
     if(k.W == W && k.H == H && k.bd == bd && k.R == R)
     {
       if(tile_w) { *tile_w = 128; }
-      if(tile_h) { *tile_h = 4 * kv.second->wy; }
+      if(tile_h) { *tile_h = cps_tile_height(kv.second->wy); }
       if(rows) { *rows = 4; }
       return true;
     }

@@ -49,6 +49,9 @@ struct CpsArgs
   uint32_t       clip;
   int32_t        wi[3];        // search weights
   float          wf[3];
+  int32_t        gmax[3];      // bound of |GCD| per component
+  int32_t        key_mid;      // 4:2:0 form: mid value and key bias (set when the pair is described)
+  uint32_t       key_bias;
   const PairOut* gcd_src;      // gcd + flags
   uint32_t*      rows;         // [2][H][3], zeroed, 32-bit wrap-around sums
   void*          scp0;         // In0 resampled (T2R search result), planar 3 x W*H, may be null
@@ -200,7 +203,8 @@ struct CpsPairPlan
   size_t   smem;        // dynamic shared memory of the pair alone
 };
 size_t      cps_desc_bytes();
-int         cps_pick_wy(int R, int esz, int sx, int sy);   // warps per tile column: 8 (128x32) or 4 (128x16), 0 = none
+// tile form: kCpsForm420 for 4:2:0, else warps per tile column: 8 (128x32) or 4 (128x16); 0 = none
+int         cps_pick_wy(int R, int esz, int sx, int sy);
 bool        cps_tile_fits(int R, int wy, int esz, int sx, int sy);
 cudaError_t cps_describe(void* desc, const CpsArgs& a, int R, int esz, int wy, CpsPairPlan* plan);
 cudaError_t launch_cps_multi(const void* d_descs, const int32_t* d_prefix, int npairs, int ntiles, int R, int wy,
@@ -208,5 +212,12 @@ cudaError_t launch_cps_multi(const void* d_descs, const int32_t* d_prefix, int n
 
 // Exactness check of the fp32 key path for a given bit depth, weights and GCD clip range.
 bool cps_fp32_exact(int32_t maxv, const int32_t w[3], const int32_t maxdiff[3]);
+// The same for the integer keys of the 4:2:0 form (qmiv_cps420.cu), with the constants its keys use.
+bool cps_shared_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[3], uint32_t* bias, int32_t* mid);
+// ... for the form a picture of these chroma shifts is searched with.
+bool cps_key_exact(int R, int sx, int sy, int32_t maxv, const int32_t w[3], const int32_t maxdiff[3]);
+// Tile form 1 is the 4:2:0 form; the others are the warps of a tile column.
+constexpr int kCpsForm420 = 1;
+inline int cps_tile_height(int wy) { return wy == kCpsForm420 ? 16 : 4 * wy; }
 
 }  // namespace qmiv

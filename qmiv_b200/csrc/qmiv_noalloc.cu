@@ -75,7 +75,7 @@ qmiv_status enqueue_static(char* base, const Shape& S, const qmiv_params& prm, c
   for(int c = 0; c < 3; c++) { ra.rows[c] = pa.rows[c]; ra.mult[c] = c ? (1 << (S.sx + S.sy)) : 1; }
   ra.area = (int64_t)S.W * S.H; ra.maxv = S.maxv;
   for(int c = 0; c < 4; c++) { ra.maxdiff[c] = maxdiff[c]; }
-  ra.need_gcd = search; ra.fp32_ok = cps_fp32_exact(S.maxv, prm.cws, maxdiff);
+  ra.need_gcd = search; ra.fp32_ok = cps_key_exact(prm.search_range, S.sx, S.sy, S.maxv, prm.cws, maxdiff);
   ra.clip_on = prm.invalid_pel_action == QMIV_PEL_CNCL;
   ra.row_sd = row_sd; ra.row_ssd = row_ssd; ra.out = dout;
   QMIV_CUDA(launch_reduce(ra, s));
@@ -84,7 +84,7 @@ qmiv_status enqueue_static(char* base, const Shape& S, const qmiv_params& prm, c
   {
     CpsArgs ca{};
     ca.in0 = in0; ca.in1 = in1; ca.W = S.W; ca.H = S.H; ca.maxv = S.maxv; ca.clip = clip;
-    for(int c = 0; c < 3; c++) { ca.wi[c] = prm.cws[c]; ca.wf[c] = (float)prm.cws[c]; }
+    for(int c = 0; c < 3; c++) { ca.wi[c] = prm.cws[c]; ca.wf[c] = (float)prm.cws[c]; ca.gmax[c] = maxdiff[c]; }
     ca.gcd_src = dout; ca.rows = cps; ca.scp0 = nullptr; ca.scp1 = nullptr;
     QMIV_CUDA(launch_cps<T>(ca, prm.search_range, s));
   }

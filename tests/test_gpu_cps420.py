@@ -1,0 +1,70 @@
+"""The 4:2:0 corresponding-pixel-shift search against the C restatement where its tiles, keys and paths
+change: pictures smaller than a tile, one sample past a tile edge, every search range, the largest bit
+depth of the integer keys and the depths past it, invalid samples, planes TMA cannot take."""
+import numpy as np
+import pytest
+
+import oracle
+import qmiv_b200
+from qmiv_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(2, 2), (10, 8), (126, 14), (128, 16), (130, 18), (262, 34)]
+
+
+def _check(qctx, oracle_lib, shape, f0, f1, dev, metrics=None, **kw):
+    W, H, bd, R = shape
+    metrics = metrics or oracle.IVPSNR | (oracle.IVSSIM if min(W, H) >= 8 else 0) | (oracle.IVMSSSIM if min(W, H) >= 32 else 0)
+    exp = oracle_lib.compute_pair(oracle.make_params(W, H, bd, 420, search_range=R), f0, f1, metrics)
+    with qmiv_b200.Calc(qctx, W, H, bd, 420, search_range=R, **kw) as calc:
+        got = calc.compute(dev(f0), dev(f1), metrics)
+    assert {k: got[k] for k in exp} == exp
+
+
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("bd,R", [(8, 1), (8, 2), (10, 2), (10, 3), (8, 4), (10, 5), (11, 4), (12, 2), (12, 3), (14, 2)])
+def test_tiles_keys_and_ranges(size, bd, R, qctx, oracle_lib):
+    f0, f1 = synth.make_pair(*size, bd, seed=7 * bd + R, shift_range=R, texture_sigma=40.0, offset=(3, -2, 2))
+    _check(qctx, oracle_lib, (*size, bd, R), f0, f1, lambda f: f)
+
+
+@pytest.mark.parametrize("size", SIZES[1:])
+@pytest.mark.parametrize("bd,top", [(8, 255), (10, 1023), (12, 4095)])
+def test_extreme_samples(size, bd, top, qctx, oracle_lib):
+    """Only the smallest and largest sample values: the widest keys, equal errors everywhere, clipped SCP samples."""
+    rng = np.random.default_rng(bd)
+    dt = np.uint8 if bd == 8 else np.uint16
+    f = [tuple((rng.integers(0, 2, (size[1] >> s, size[0] >> s)) * top).astype(dt) for s in (0, 1, 1)) for _ in range(2)]
+    _check(qctx, oracle_lib, (*size, bd, 2), f[0], f[1], lambda x: x)
+
+
+@pytest.mark.parametrize("size,R", [((130, 18), 2), ((262, 34), 3)])
+def test_samples_above_the_maximum(size, R, qctx, oracle_lib):
+    """SKIP searches them as they are (literal int32 arithmetic); CNCL clips them first."""
+    f0, f1 = synth.make_pair(*size, 10, seed=3)
+    hot = [tuple(p.copy() for p in f) for f in (f0, f1)]
+    hot[0][0][5, 7] = 40000
+    hot[1][1][3, 2] = 65535
+    _check(qctx, oracle_lib, (*size, 10, R), hot[0], hot[1], lambda f: f, metrics=oracle.IVPSNR,
+           invalid_pel_action=qmiv_b200.PEL_SKIP)   # window moments of samples above 14 bits wrap and are not compared
+    clipped = [tuple(np.minimum(p, 1023) for p in f) for f in hot]
+    exp = oracle_lib.compute_pair(oracle.make_params(*size, 10, 420, search_range=R), *clipped, oracle.IVPSNR | oracle.IVSSIM)
+    with qmiv_b200.Calc(qctx, *size, 10, 420, search_range=R, invalid_pel_action=qmiv_b200.PEL_CNCL) as calc:
+        got = calc.compute(*hot, oracle.IVPSNR | oracle.IVSSIM)
+    assert all(got[k] == exp[k] for k in exp if k != "invalid_pel")
+
+
+@pytest.mark.parametrize("bd", [8, 10])
+def test_planes_without_tma(bd, qctx, oracle_lib):
+    """Device planes whose pitch is no multiple of 16 bytes are loaded sample by sample."""
+    import torch
+    def dev(frame):
+        out = []
+        for p in frame:
+            t = torch.zeros(p.shape[0], p.shape[1] + 3, dtype=torch.uint8 if bd == 8 else torch.uint16, device="cuda")
+            t[:, :p.shape[1]] = torch.from_numpy(np.ascontiguousarray(p)).cuda()
+            out.append(t[:, :p.shape[1]])
+        return tuple(out)
+    f0, f1 = synth.make_pair(262, 50, bd, seed=11)
+    _check(qctx, oracle_lib, (262, 50, bd, 2), f0, f1, dev)

@@ -234,3 +234,34 @@ def test_mask_byte_count_and_or_flag():
             if rng.random() < 0.5:
                 x[rng.integers(0, x.size)] = rng.integers(maxv + 1, 1 << 16)
             assert (np.bitwise_or.reduce(x) > maxv) == (x.max() > maxv)
+
+
+@pytest.mark.parametrize("bd,w,R", [(8, (4, 1, 1), 5), (10, (4, 1, 1), 2), (11, (4, 1, 1), 4), (12, (4, 1, 1), 2), (9, (6, 2, 3), 3)])
+def test_shared_chroma_keys_order_like_int32_errors(bd, w, R):
+    """The 4:2:0 search's key in uint32: luma cross term + (luma square + chroma part + raster code), samples
+    relative to the mid value and a bias for the dropped test terms, orders candidates as (error, raster
+    index); the extremes of the ranges included."""
+    rng = np.random.default_rng(100 * bd + R)
+    maxv, D, n = (1 << bd) - 1, 2 * R + 1, 4000
+    g = int(0.01 * maxv + 0.5)
+    K = 32 if R <= 2 else 64 if R == 3 else 128
+    m = (maxv + 1) // 2
+    wi = np.array(w, np.int64)
+    lo, hi = int((wi * (m + g) ** 2).sum()), int((wi * (m * m + 2 * (m + g) * m)).sum())
+    assert K * (lo + hi) + (3 + 2 * R) * D + 3 + 2 * R < (1 << 32) - 1          # the host's condition
+    s = rng.integers(-g, maxv + g + 1, (n, 3)).astype(np.int64)
+    r = rng.integers(0, maxv + 1, (n, D * D, 3)).astype(np.int64)
+    s[:200] = rng.choice([-g, maxv + g], (200, 3))
+    r[:200] = rng.choice([0, maxv], (200, D * D, 3))
+    r[:, 5] = r[:, 2]
+    best = np.argmin(((s[:, None] - r) ** 2 * wi).sum(-1), axis=1)
+    u = lambda v: np.asarray(v, np.int64).astype(np.uint32)
+    k = np.arange(D * D)
+    for i, j in ((0, 0), (3, 3)):                                                 # corner pixels of a 4x4 block
+        code = (k // D + i) * D + k % D + j
+        sc, rc = s - m, r - m
+        P = u(K * (wi[1] * rc[..., 1] ** 2 + wi[2] * rc[..., 2] ** 2 + lo)) - u(2 * K * (wi[1] * sc[:, None, 1] * rc[..., 1] + wi[2] * sc[:, None, 2] * rc[..., 2]))
+        t = u(K * wi[0] * rc[..., 0] ** 2) + P + u(code)
+        key = u(-2 * K * wi[0] * sc[:, None, 0]) * u(rc[..., 0]) + t
+        assert np.array_equal(np.argmin(key, axis=1), best)
+        assert np.array_equal((key.min(axis=1) - u(i * D + j)) & np.uint32(K - 1), best)
