@@ -506,7 +506,7 @@ qmiv_status PairPipeline::enqueue_ssim_gen(const Img& in0, const Img& in1, const
       J = SsimGenJob{};
       J.a = a; J.b = b; J.comp = c; J.W = S.W >> scale; J.H = S.H >> scale;
       J.x0 = gfirst_; J.y0 = gfirst_; J.nx = gnx_[scale]; J.ny = gny_[scale];
-      J.calc_l = calc_l; J.clip = clip; J.esz = (int32_t)S.esz; J.C1 = C1_; J.C2 = C2_;
+      J.calc_l = calc_l; J.clip = clip; J.esz = (int32_t)S.esz; J.small_range = S.maxv < 0x4000; J.flags = &out_.as<PairOut>()->flags; J.C1 = C1_; J.C2 = C2_;
       J.win = win_.as<double>() + (size_t)ga.njobs * wstride;
       SsimPoolJob& P = rows.job[rows.njobs];
       P = SsimPoolJob{};

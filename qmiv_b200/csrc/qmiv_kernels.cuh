@@ -109,6 +109,8 @@ struct SsimGenJob
   int32_t  calc_l;
   uint32_t clip;       // conceal: samples above are clipped (65535 = no clipping)
   int32_t  esz;        // bytes per sample of a and b
+  int32_t  small_range;   // the bit depth's maximum is below 2^14
+  const int32_t* flags;   // PairOut::flags: bits 0 and 1 = samples above the maximum
   double   C1, C2;
   double*  win;        // [ceil(ny / 32)][nx][32] (pool_win_elems)
 };

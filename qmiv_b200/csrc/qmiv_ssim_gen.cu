@@ -11,8 +11,12 @@
 //     Gaussian integer 8 / 16 (xStructSimSTD.cpp:353-419), averaged 8 / 16 / 32 (:420-461) x (1 / N^2)
 // Integer sums stay below 2^53 for 16-bit samples (65535^2 * 2^18 < 2^51), so they are formed exactly in
 // double with fused multiply-adds in any order; the float Gaussian sums keep the reference's order and
-// roundings (separate multiply and add). The window formula uses separately rounded operations in the
-// reference's order, so every window value equals the portable reference's bit for bit.
+// roundings (separate multiply and add). For samples below 2^14 every product there is exact (a sample
+// product has at most 28 bits, a float coefficient 24: 52 bits fit a double's 53), so a fused multiply-add,
+// which rounds the sum alone, gives the same double in half the FP64 instructions; pictures with larger
+// samples (15 and 16 bits, the 65535 margin, invalid samples) keep the separate form. The window formula
+// uses separately rounded operations in the reference's order, so every window value equals the portable
+// reference's bit for bit.
 //
 // Three window kernels, all staging the samples a CTA's windows read in shared memory, both pictures
 // packed (a | b << 16) after clipping and margin extension:
@@ -32,7 +36,7 @@ namespace qmiv {
 
 namespace {
 
-enum { kGenFlt = 0, kGenInt = 1, kGenAvg = 2 };
+enum { kGenFlt = 0, kGenInt = 1, kGenAvg = 2, kGenFltFma = 3 };   // kGenFltFma: kGenFlt with exact products
 
 // window coefficients, row-major dy * N + dx
 constexpr int kCoefFlt11 = 0, kCoefInt11 = 121, kCoefInt8 = 242, kCoefInt16 = 306, kCoefTotal = 562;
@@ -76,8 +80,22 @@ void build_coefs(double* c)
   for(int y = 0; y < 16; y++) { for(int x = 0; x < 16; x++) { c[kCoefInt16 + 16 * y + x] = gauss_int(16, y, x); } }
 }
 
-// exact double of a 16-bit integer: 2^52 + v has a unit ulp
-__device__ __forceinline__ double u16_to_f64(uint32_t v) { return dsub(__hiloint2double(0x43300000, (int)v), 4503599627370496.0); }
+// The five values of a packed sample pair (a | b << 16). The samples are converted on the conversion unit,
+// which runs beside the FP64 pipe that the sums keep busy; the products, exact below 2^32, are FP64 (all
+// five on the conversion unit measured 922 us against 909 in the launch below, none on it 962).
+struct GenSample { double R, T, RR, TT, RT; };
+__device__ __forceinline__ GenSample gen_sample(uint32_t v)
+{
+  const double R = __uint2double_rn(v >> 16), T = __uint2double_rn(v & 0xffffu);
+  return GenSample{ R, T, dmul(R, R), dmul(T, T), dmul(R, T) };
+}
+
+// Whether every product of the float Gaussian sums is exact: all samples of the job, margin included,
+// are below 2^14 (bytes, or clipped, or checked by the prepass).
+__device__ __forceinline__ bool gen_exact_products(const SsimGenJob& J, int border)
+{
+  return border != QMIV_BRD_CONSTANT && (J.esz == 1 || J.clip < 0x4000u || (J.small_range && (*J.flags & 3) == 0));
+}
 
 // position of sample i of a length-n line after margin extension; in = false for the constant modes
 __device__ __forceinline__ int brd_map(int i, int n, int border, bool& in)
@@ -148,7 +166,7 @@ __device__ __forceinline__ double gen_window(const double (&m)[5], double inv, d
 {
   // m: sums of R, T, R^2, T^2, R*T (R = "Ref" = b, T = "Tst" = a)
   double ar, at, var_r, var_t, cov;
-  if(MODE == kGenFlt)                                         // xStructSimSTD.cpp:41-45
+  if(MODE == kGenFlt || MODE == kGenFltFma)                   // xStructSimSTD.cpp:41-45
   {
     ar = m[0]; at = m[1];
     var_r = dsub(m[2], dmul(ar, ar));
@@ -173,9 +191,8 @@ __device__ __forceinline__ double gen_window(const double (&m)[5], double inv, d
 // column x0 + l of window row y0 + w. With stride S > 1 the tile's columns are stored by phase (column c
 // at (c % S) * cw + c / S), so the 32 lanes of a warp read 32 consecutive words.
 template <int MODE, int N, int K>
-__global__ void __launch_bounds__(128) k_ssim_gen(const __grid_constant__ SsimGenArgs a)
+__device__ __forceinline__ void gen_body(const SsimGenArgs& a, uint32_t* tile)   // tile [th][S * cw], sample a | b << 16
 {
-  extern __shared__ uint32_t tile[];                          // [th][S * cw], sample a | b << 16
   const SsimGenJob& J = a.job[blockIdx.z];
   const int S = a.S, WY = blockDim.y, lane = threadIdx.x, w = threadIdx.y;
   const int wx0 = blockIdx.x * 32, wy0 = blockIdx.y * WY * K;
@@ -218,8 +235,8 @@ __global__ void __launch_bounds__(128) k_ssim_gen(const __grid_constant__ SsimGe
     for(int dx = 0; dx < N; dx++)
     {
       const uint32_t v = rowp[co[dx]];
-      const double T = u16_to_f64(v & 0xffffu), R = u16_to_f64(v >> 16);
-      const double RR = dmul(R, R), TT = dmul(T, T), RT = dmul(R, T);   // exact (< 2^32)
+      const GenSample g = gen_sample(v);
+      const double R = g.R, T = g.T, RR = g.RR, TT = g.TT, RT = g.RT;
       #pragma unroll
       for(int k = 0; k < K; k++)
       {
@@ -238,7 +255,7 @@ __global__ void __launch_bounds__(128) k_ssim_gen(const __grid_constant__ SsimGe
             acc[k][2] = dadd(acc[k][2], dmul(RR, C)); acc[k][3] = dadd(acc[k][3], dmul(TT, C));
             acc[k][4] = dadd(acc[k][4], dmul(RT, C));
           }
-          else                                                // exact integers
+          else                                                // exact products
           {
             acc[k][0] = __fma_rn(R, C, acc[k][0]); acc[k][1] = __fma_rn(T, C, acc[k][1]);
             acc[k][2] = __fma_rn(RR, C, acc[k][2]); acc[k][3] = __fma_rn(TT, C, acc[k][3]);
@@ -261,6 +278,14 @@ __global__ void __launch_bounds__(128) k_ssim_gen(const __grid_constant__ SsimGe
   }
 }
 
+template <int MODE, int N, int K>
+__global__ void __launch_bounds__(128) k_ssim_gen(const __grid_constant__ SsimGenArgs a)
+{
+  extern __shared__ uint32_t tile[];
+  if(MODE == kGenFlt && gen_exact_products(a.job[blockIdx.z], a.border)) { gen_body<kGenFltFma, N, K>(a, tile); }
+  else { gen_body<MODE, N, K>(a, tile); }
+}
+
 // Row-walking form for strides 1, 2 and 4 (the original paper's and the app's default stride): lane l of
 // warp w evaluates the K windows x0 + l K .. x0 + l K + K - 1 of window rows w, w + 4, ... of the CTA.
 // For each window row it walks the N input rows in order; in input row dy, input column j of the lane's
@@ -269,12 +294,15 @@ __global__ void __launch_bounds__(128) k_ssim_gen(const __grid_constant__ SsimGe
 // instruction is spent on a tap a window does not have, and each window still receives its taps in
 // dy-major, dx-minor order. The N coefficients of row dy are loaded once per row. The tile's columns are
 // stored by phase modulo K S, so the lanes of a warp read consecutive words.
+// What bounds it: the FP64 pipe (605 multiply-adds per Gaussian window, 3 products per staged sample and
+// window row, two correctly rounded divisions per window). Float Gaussian, stride 1, 1920x1080 8-bit, three
+// evaluations of three components: 1641 us with separate products and sums, 909 fused, 871 with the launch
+// shape of gen_plan_rows.
 template <int MODE, int N, int K, int S>
-__global__ void __launch_bounds__(128) k_ssim_gen_rows(const __grid_constant__ SsimGenArgs a)
+__device__ __forceinline__ void gen_rows_body(const SsimGenArgs& a, uint32_t* tile)   // tile [th][KS * cw], sample a | b << 16
 {
   constexpr int KS = K * S;
   constexpr int J = (K - 1) * S + N;                          // input columns of one lane's windows
-  extern __shared__ uint32_t tile[];                          // [th][KS * cw], sample a | b << 16
   const SsimGenJob& Jb = a.job[blockIdx.z];
   const int lane = threadIdx.x, w = threadIdx.y;
   const int WR = a.wr;                                        // window rows per CTA
@@ -312,8 +340,8 @@ __global__ void __launch_bounds__(128) k_ssim_gen_rows(const __grid_constant__ S
       for(int j = 0; j < J; j++)
       {
         const uint32_t v = rowp[(j % KS) * cw + j / KS];
-        const double T = u16_to_f64(v & 0xffffu), R = u16_to_f64(v >> 16);
-        const double RR = dmul(R, R), TT = dmul(T, T), RT = dmul(R, T);   // exact (< 2^32)
+        const GenSample g = gen_sample(v);
+        const double R = g.R, T = g.T, RR = g.RR, TT = g.TT, RT = g.RT;
         #pragma unroll
         for(int k = 0; k < K; k++)
         {
@@ -330,7 +358,7 @@ __global__ void __launch_bounds__(128) k_ssim_gen_rows(const __grid_constant__ S
             acc[k][2] = dadd(acc[k][2], dmul(RR, C[dx])); acc[k][3] = dadd(acc[k][3], dmul(TT, C[dx]));
             acc[k][4] = dadd(acc[k][4], dmul(RT, C[dx]));
           }
-          else                                                // exact integers
+          else                                                // exact products
           {
             acc[k][0] = __fma_rn(R, C[dx], acc[k][0]); acc[k][1] = __fma_rn(T, C[dx], acc[k][1]);
             acc[k][2] = __fma_rn(RR, C[dx], acc[k][2]); acc[k][3] = __fma_rn(TT, C[dx], acc[k][3]);
@@ -347,6 +375,14 @@ __global__ void __launch_bounds__(128) k_ssim_gen_rows(const __grid_constant__ S
       if(wx + k < Jb.nx) { out[(size_t)(wx + k) * 32] = gen_window<MODE, N>(acc[k], a.inv, Jb.C1, Jb.C2, Jb.calc_l != 0); }
     }
   }
+}
+
+template <int MODE, int N, int K, int S>
+__global__ void __launch_bounds__(128) k_ssim_gen_rows(const __grid_constant__ SsimGenArgs a)
+{
+  extern __shared__ uint32_t tile[];
+  if(MODE == kGenFlt && gen_exact_products(a.job[blockIdx.z], a.border)) { gen_rows_body<kGenFltFma, N, K, S>(a, tile); }
+  else { gen_rows_body<MODE, N, K, S>(a, tile); }
 }
 
 // Averaged windows (regular 11x11 and block 8 / 16 / 32) at strides 1, 2 and 4 by box sums. Their five
@@ -479,8 +515,21 @@ struct GenPlan
 };
 
 // Windows per lane of the row-walking form (strides 1, 2, 4): enough that a loaded sample feeds several
-// windows, few enough that the tile of 32 K windows stays small.
+// windows, few enough that the tile of 32 K windows stays small. The 11x11 Gaussian windows at stride 1
+// exist with 8 and 6 windows per lane; gen_plan_rows picks.
 constexpr int rows_k(int S, int N) { return S == 1 ? 8 : (S == 2 || N < 32) ? 4 : 2; }
+constexpr int rows_k_alt(int MODE, int S, int N) { return S == 1 && N == 11 && MODE != kGenAvg ? 6 : 0; }
+
+// Tile of the row-walking form with K windows per lane and wr window rows per CTA.
+void rows_tile(int N, int S, int K, int wr, GenPlan& p)
+{
+  const int KS = K * S;
+  p.K = K; p.WY = 4; p.wr = wr;
+  p.tw = (32 * K - 1) * S + N;
+  p.th = (wr - 1) * S + N;
+  p.cw = (p.tw + KS - 1) / KS;
+  p.smem = (size_t)p.th * KS * p.cw * sizeof(uint32_t);
+}
 
 // Launch shape of either form: the row-walking form for strides 1, 2 and 4 with as many window rows per
 // CTA as fit 48 KB of tile; one window per thread otherwise (every tap of a thread's window is its own,
@@ -489,15 +538,9 @@ bool gen_plan(int N, int S, GenPlan& p)
 {
   if(S == 1 || S == 2 || S == 4)
   {
-    const int K = rows_k(S, N), KS = K * S;
-    p.K = K; p.WY = 4;
-    p.tw = (32 * K - 1) * S + N;
-    p.cw = (p.tw + KS - 1) / KS;
     for(int wr = 32; wr >= 4; wr >>= 1)
     {
-      p.wr = wr;
-      p.th = (wr - 1) * S + N;
-      p.smem = (size_t)p.th * KS * p.cw * sizeof(uint32_t);
+      rows_tile(N, S, rows_k(S, N), wr, p);
       if(p.smem <= kGenSmemPreferred) { return true; }
     }
     return p.smem <= kGenSmemMax;
@@ -513,7 +556,43 @@ bool gen_plan(int N, int S, GenPlan& p)
 template <int MODE, int N, int S>
 cudaError_t gen_attr_rows()
 {
-  return cudaFuncSetAttribute(k_ssim_gen_rows<MODE, N, rows_k(S, N), S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGenSmemMax);
+  cudaError_t e = cudaFuncSetAttribute(k_ssim_gen_rows<MODE, N, rows_k(S, N), S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGenSmemMax);
+  if constexpr(rows_k_alt(MODE, S, N) != 0)
+  {
+    if(e == cudaSuccess) { e = cudaFuncSetAttribute(k_ssim_gen_rows<MODE, N, rows_k_alt(MODE, S, N), S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGenSmemMax); }
+  }
+  return e;
+}
+
+// Windows per lane and window rows per CTA of the Gaussian windows at stride 1, whose FP64 sums fill the
+// launch: the shape with the least work by waves of CTAs, counting a CTA's FP64 instructions per warp
+// (K (N N 5) multiply-adds and 3 products per staged sample and window row) and a share of its staging. A
+// fixed shape of 8 windows x 32 rows left a 1920x1080 picture's fifth wave nearly empty and half of its last
+// column of tiles idle.
+template <int MODE, int N>
+void gen_plan_rows(const SsimGenArgs& a, GenPlan& p)
+{
+  constexpr int ks[2] = { rows_k(1, N), rows_k_alt(MODE, 1, N) };
+  int dev = 0, sms = 1;
+  if(cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) { return; }
+  double least = 0.0;
+  for(int c = 0; c < 2; c++)
+  {
+    const int K = ks[c];
+    for(int wr = 4; wr <= 32; wr += 4)
+    {
+      GenPlan q;
+      rows_tile(N, 1, K, wr, q);
+      if(q.smem > kGenSmemPreferred) { break; }
+      const int occ = 4;   // by registers (at most 128) and by shared memory alike
+      long ctas = 0;
+      for(int k = 0; k < a.njobs; k++) { ctas += (long)((a.job[k].nx + 32 * K - 1) / (32 * K)) * ((a.job[k].ny + wr - 1) / wr); }
+      const long waves = (ctas + (long)sms * occ - 1) / ((long)sms * occ);
+      const double cta = (wr / 4) * (double)N * ((K - 1 + N) * 3 + K * N * 5) + (double)q.th * q.tw / 128.0 * 12.0;
+      const double cost = waves * cta;
+      if(least == 0.0 || cost < least) { least = cost; p = q; }
+    }
+  }
 }
 
 template <int MODE, int N>
@@ -553,12 +632,25 @@ cudaError_t gen_configure()
 }
 
 template <int MODE, int N>
-cudaError_t gen_launch_k(const SsimGenArgs& a, const GenPlan& p, int S, int maxnx, int maxny, cudaStream_t s)
+cudaError_t gen_launch_k(SsimGenArgs& a, GenPlan p, int S, int maxnx, int maxny, cudaStream_t s)
 {
+  if constexpr(rows_k_alt(MODE, 1, N) != 0)
+  {
+    if(S == 1) { gen_plan_rows<MODE, N>(a, p); }
+  }
+  a.tw = p.tw; a.th = p.th; a.cw = p.cw; a.wr = p.wr;
   const dim3 block(32, p.WY);
   if(p.wr > 0)
   {
     const dim3 grid((maxnx + 32 * p.K - 1) / (32 * p.K), (maxny + p.wr - 1) / p.wr, a.njobs);
+    if constexpr(rows_k_alt(MODE, 1, N) != 0)
+    {
+      if(S == 1 && p.K == rows_k_alt(MODE, 1, N))
+      {
+        k_ssim_gen_rows<MODE, N, rows_k_alt(MODE, 1, N), 1><<<grid, block, p.smem, s>>>(a);
+        return cudaGetLastError();
+      }
+    }
     if(S == 1) { k_ssim_gen_rows<MODE, N, rows_k(1, N), 1><<<grid, block, p.smem, s>>>(a); }
     else if(S == 2) { k_ssim_gen_rows<MODE, N, rows_k(2, N), 2><<<grid, block, p.smem, s>>>(a); }
     else { k_ssim_gen_rows<MODE, N, rows_k(4, N), 4><<<grid, block, p.smem, s>>>(a); }
@@ -631,7 +723,7 @@ cudaError_t launch_ssim_gen(SsimGenArgs& a, int mode, int N, int S, int border, 
     if(J.nx < 1 || J.ny < 1 || !J.win || (J.esz != 1 && J.esz != 2)) { return cudaErrorInvalidValue; }
     maxnx = max(maxnx, J.nx); maxny = max(maxny, J.ny);
   }
-  a.S = S; a.border = border; a.tw = p.tw; a.th = p.th; a.cw = p.cw; a.wr = p.wr;
+  a.S = S; a.border = border;
   const bool box = S == 1 || S == 2 || S == 4;                      // averaged windows by box sums
   switch(mode)
   {
