@@ -880,7 +880,7 @@ cudaError_t launch_cps_multi(const void* d_descs, const int32_t* d_prefix, int n
   cudaError_t e = cudaGetDevice(&dev);
   if(e != cudaSuccess) { return e; }
   const CpsKernelArgs* d = static_cast<const CpsKernelArgs*>(d_descs);
-  if(wy == kCpsForm420) { return cps420_launch_multi(d, d_prefix, npairs, ntiles, R, esz, s); }
+  if(wy == kCpsForm420) { return cps420_launch_multi(d, d_prefix, npairs, ntiles, R, esz, 0, s); }
   auto go = [&](auto tag) -> cudaError_t {
     using T = decltype(tag);
     switch(R)

@@ -31,6 +31,7 @@ struct CpsGeomArgs
 struct alignas(64) CpsKernelArgs
 {
   CUtensorMap map[2][3];       // [picture][plane]
+  CUtensorMap mask_map;        // masked 4:2:0 search
   CpsArgs     a;
   CpsGeomArgs g;
 };
@@ -137,6 +138,6 @@ bool        cps420_fits(int R, int esz);
 int         cps420_tiles(int W, int H);
 cudaError_t cps420_describe(CpsKernelArgs& k, int R, int esz, CpsPairPlan* plan);
 cudaError_t cps420_launch(const CpsKernelArgs& k, int R, int esz, cudaStream_t s);
-cudaError_t cps420_launch_multi(const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, int R, int esz, cudaStream_t s);
+cudaError_t cps420_launch_multi(const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, int R, int esz, int mesz, cudaStream_t s);
 
 }  // namespace qmiv

@@ -42,11 +42,17 @@
 // with double-buffered boxes measure 883 us with moments but 485 with stored pictures, so the raw boxes
 // are double-buffered only where three CTAs do not fit.
 //
+// With a mask (mask mode) the same tiles also bring the mask's samples; masked reference samples are staged
+// above every real key and the winners' squared differences are weighted by the test pixels' mask values.
+// 4096x2048, 10 bits, 8-bit mask: 193 us by the fp32-key kernel (one pixel column per thread, tiles staged
+// sample by sample, no copies in flight) -> 115; 8 pairs of 1920x1080, 8 bits: 383 -> 244.
+//
 // Pictures with samples above the maximum (SKIP and WARN actions) and parameters whose keys do not fit
 // take the literal int32 search below (the SSE path's wrap-around arithmetic) in the same frame.
 #include "qmiv_cps.cuh"
 
 #include <cstring>
+#include <type_traits>
 
 namespace qmiv {
 
@@ -54,12 +60,19 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// Geometry of one search range and sample type; every size is known at compile time.
-template <int R, typename T>
+// K = 2^key_bits: above the largest raster index
+__host__ __device__ constexpr int key_bits(int R) { return R <= 2 ? 5 : (R == 3 ? 6 : 7); }
+
+// Sample type of the mask of a search without one
+struct NoMask { };
+
+// Geometry of one search range, sample type and mask sample type; every size is known at compile time.
+template <int R, typename T, typename TM = NoMask>
 struct Geo420
 {
+  static constexpr bool MASK = !std::is_same<TM, NoMask>::value;
   static constexpr int D = 2 * R + 1;
-  static constexpr int KB = R <= 2 ? 5 : (R == 3 ? 6 : 7);         // key bits of the raster code
+  static constexpr int KB = key_bits(R);                           // key bits of the raster code
   static constexpr uint32_t K = 1u << KB;
   static_assert(D * D <= (1 << KB), "raster codes fit");
   static constexpr int TW = 128, TH = 16, NT = 256;
@@ -75,8 +88,11 @@ struct Geo420
   // raw boxes of one picture: luma, Cb, Cr
   static constexpr uint32_t OFFU = align_up(BHL * PLB, kAlign), OFFV = OFFU + align_up(BHC * PCB, kAlign);
   static constexpr uint32_t PIC = OFFV + align_up(BHC * PCB, kAlign);
-  static constexpr uint32_t STAGE = 2 * PIC;
-  static constexpr uint32_t TX = 2u * (uint32_t)(BHL * PLB + 2 * BHC * PCB);
+  // the mask's box behind both pictures'
+  static constexpr int MESZ = (int)sizeof(TM), AXM = 16 / MESZ, BWM = (int)align_up(AXM + TW + R, AXM);
+  static constexpr uint32_t OFFM = 2 * PIC;
+  static constexpr uint32_t STAGE = OFFM + (MASK ? align_up(BHL * BWM * MESZ, kAlign) : 0u);
+  static constexpr uint32_t TX = 2u * (uint32_t)(BHL * PLB + 2 * BHC * PCB) + (MASK ? (uint32_t)(BHL * BWM * MESZ) : 0u);
   // staged rows, in 16-byte pairs of samples
   static constexpr int HALF = (SW / 2 + 1) / 2, LPP = 2 * HALF;    // luma: even pairs, then odd pairs
   static constexpr int CPP = CW / 2;                               // chroma
@@ -103,10 +119,10 @@ struct Pair420
   int                  tile;
 };
 
-template <int R, typename T>
+template <int R, typename T, typename TM>
 __device__ __forceinline__ void issue_tile420(const CpsKernelArgs& k, bool new_maps, unsigned char* raw, uint64_t* bar, int t)
 {
-  using G = Geo420<R, T>;
+  using G = Geo420<R, T, TM>;
   const int x0 = (t % k.g.ntx) * G::TW, y0 = (t / k.g.ntx) * G::TH;
   if(new_maps)   // the first use of a pair's tensor maps, which the host copied to global memory
   {
@@ -116,6 +132,7 @@ __device__ __forceinline__ void issue_tile420(const CpsKernelArgs& k, bool new_m
       #pragma unroll
       for(int c = 0; c < 3; c++) { fence_tensormap_acquire(&k.map[f][c]); }
     }
+    if(G::MASK) { fence_tensormap_acquire(&k.mask_map); }
   }
   mbar_expect_tx(bar, G::TX);
   #pragma unroll
@@ -126,46 +143,76 @@ __device__ __forceinline__ void issue_tile420(const CpsKernelArgs& k, bool new_m
     tma_load_2d(p + G::OFFU, &k.map[f][1], (x0 >> 1) - G::AX, (y0 - R) >> 1, bar);
     tma_load_2d(p + G::OFFV, &k.map[f][2], (x0 >> 1) - G::AX, (y0 - R) >> 1, bar);
   }
+  if(G::MASK) { tma_load_2d(raw + G::OFFM, &k.mask_map, x0 - G::AXM, y0 - R, bar); }
 }
 
-// The same boxes by plain loads, for frames whose address or pitch TMA cannot take (samples outside
-// the picture stay unwritten: complete_halo fills them).
-template <int R, typename T>
+// One box by plain loads, for planes whose address or pitch TMA cannot take (samples outside the picture
+// stay unwritten: complete_halo fills them). xs, ys: picture position of the box; pw, ph: plane size.
+template <typename S, int NT>
+__device__ __forceinline__ void load_box(const S* src, int pitch, S* dst, int bw, int bh, int xs, int ys, int pw, int ph)
+{
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for(int r = warp; r < bh; r += NT / 32)
+  {
+    const int gy = ys + r;
+    if(gy < 0 || gy >= ph) { continue; }
+    for(int col = lane; col < bw; col += 32)
+    {
+      const int gx = xs + col;
+      if(gx >= 0 && gx < pw) { dst[r * bw + col] = __ldg(src + (size_t)gy * pitch + gx); }
+    }
+  }
+}
+
+template <int R, typename T, typename TM>
 __device__ __noinline__ void load_plain420(const CpsArgs& a, unsigned char* raw, int x0, int y0)
 {
-  using G = Geo420<R, T>;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  using G = Geo420<R, T, TM>;
   #pragma unroll 1
   for(int fc = 0; fc < 6; fc++)
   {
     const int f = fc / 3, c = fc - 3 * f;
     const Img& im = f ? a.in1 : a.in0;
-    const int pw = c ? a.W >> 1 : a.W, ph = c ? a.H >> 1 : a.H;
-    const int bw = c ? G::BWC : G::BWL, bh = c ? G::BHC : G::BHL;
-    const int xs = (c ? x0 >> 1 : x0) - G::AX, ys = c ? (y0 - R) >> 1 : y0 - R;
-    T* dst = reinterpret_cast<T*>(raw + f * G::PIC + (c == 0 ? 0u : c == 1 ? G::OFFU : G::OFFV));
-    const T* src = static_cast<const T*>(im.p[c]);
-    for(int r = warp; r < bh; r += G::NT / 32)
+    load_box<T, G::NT>(static_cast<const T*>(im.p[c]), im.pitch[c],
+                       reinterpret_cast<T*>(raw + f * G::PIC + (c == 0 ? 0u : c == 1 ? G::OFFU : G::OFFV)), c ? G::BWC : G::BWL,
+                       c ? G::BHC : G::BHL, (c ? x0 >> 1 : x0) - G::AX, c ? (y0 - R) >> 1 : y0 - R, c ? a.W >> 1 : a.W, c ? a.H >> 1 : a.H);
+  }
+  if constexpr(G::MASK)
+  {
+    load_box<TM, G::NT>(static_cast<const TM*>(a.mask), a.mask_pitch, reinterpret_cast<TM*>(raw + G::OFFM), G::BWM, G::BHL, x0 - G::AXM, y0 - R, a.W, a.H);
+  }
+}
+
+// Edge replication, in place, of a box's samples outside the picture that a candidate of a pixel inside can
+// reach. left: first column used; m: reach past the picture; inx0 .. inx1, iny0 .. iny1: the part inside.
+// Sources lie inside the picture and the box (a tile starts inside the picture) and are not written.
+template <typename S, int NT>
+__device__ __forceinline__ void replicate_box(S* p, int bw, int bh, int left, int m, int inx0, int inx1, int iny0, int iny1)
+{
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int right = min(bw, inx1 + m), rows = min(bh, iny1 + m);
+  for(int r = warp; r < rows; r += NT / 32)
+  {
+    const int sr = clampi(r, iny0, iny1 - 1);
+    const S* src = p + sr * bw;
+    S* dst = p + r * bw;
+    if(sr != r)
     {
-      const int gy = ys + r;
-      if(gy < 0 || gy >= ph) { continue; }
-      for(int col = lane; col < bw; col += 32)
-      {
-        const int gx = xs + col;
-        if(gx >= 0 && gx < pw) { dst[r * bw + col] = __ldg(src + (size_t)gy * im.pitch[c] + gx); }
-      }
+      for(int x = left + lane; x < right; x += 32) { dst[x] = src[clampi(x, inx0, inx1 - 1)]; }
+    }
+    else
+    {
+      for(int x = left + lane; x < inx0; x += 32) { dst[x] = src[inx0]; }
+      for(int x = inx1 + lane; x < right; x += 32) { dst[x] = src[inx1 - 1]; }
     }
   }
 }
 
-// Conceal clipping of the whole boxes, then edge replication, in place, of the samples outside the
-// picture that a candidate of a pixel inside can reach. Sources lie inside the picture and the box (a
-// tile starts inside the picture) and are not written by the second pass.
-template <int R, typename T>
+// Conceal clipping of the whole boxes, then the halo outside the picture.
+template <int R, typename T, typename TM>
 __device__ __noinline__ void complete_halo(const CpsArgs& a, unsigned char* raw, int x0, int y0, bool clip, bool border)
 {
-  using G = Geo420<R, T>;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  using G = Geo420<R, T, TM>;
   #pragma unroll 1
   for(int pass = clip ? 0 : 1; pass < (border ? 2 : 1); pass++)
   {
@@ -181,23 +228,14 @@ __device__ __noinline__ void complete_halo(const CpsArgs& a, unsigned char* raw,
         continue;
       }
       const int xs = (c ? x0 >> 1 : x0) - G::AX, ys = c ? (y0 - R) >> 1 : y0 - R;
-      const int inx0 = max(0, -xs), inx1 = (c ? a.W >> 1 : a.W) - xs;      // box columns / rows inside the picture
-      const int iny0 = max(0, -ys), iny1 = (c ? a.H >> 1 : a.H) - ys;
-      const int left = G::AX - m, right = min(bw, inx1 + m), rows = min(bh, iny1 + m);
-      for(int r = warp; r < rows; r += G::NT / 32)
+      replicate_box<T, G::NT>(p, bw, bh, G::AX - m, m, max(0, -xs), (c ? a.W >> 1 : a.W) - xs, max(0, -ys), (c ? a.H >> 1 : a.H) - ys);
+    }
+    if constexpr(G::MASK)
+    {
+      if(pass == 1)
       {
-        const int sr = clampi(r, iny0, iny1 - 1);
-        const T* src = p + sr * bw;
-        T* dst = p + r * bw;
-        if(sr != r)
-        {
-          for(int x = left + lane; x < right; x += 32) { dst[x] = src[clampi(x, inx0, inx1 - 1)]; }
-        }
-        else
-        {
-          for(int x = left + lane; x < inx0; x += 32) { dst[x] = src[inx0]; }
-          for(int x = inx1 + lane; x < right; x += 32) { dst[x] = src[inx1 - 1]; }
-        }
+        replicate_box<TM, G::NT>(reinterpret_cast<TM*>(raw + G::OFFM), G::BWM, G::BHL, G::AXM - R, R, max(0, G::AXM - x0), a.W - x0 + G::AXM,
+                                 max(0, R - y0), a.H - y0 + R);
       }
     }
     __syncthreads();
@@ -253,12 +291,15 @@ __device__ __forceinline__ void load_test420(const unsigned char* tst, int by, i
   for(int b = 0; b < 4; b++) { tu[b] = pu[(b >> 1) * G::BWC + (b & 1)]; tv[b] = pv[(b >> 1) * G::BWC + (b & 1)]; }
 }
 
-// raw boxes -> staged luma and chroma of both pictures
-template <int R, typename T>
+// raw boxes -> staged luma and chroma of both pictures. Under a mask a masked luma sample is staged as
+// (0, masked): its keys are masked + P + code whatever the test pixel, above every key of an unmasked one.
+template <int R, typename T, typename TM>
 __device__ __forceinline__ void stage420(const unsigned char* raw, uint4* luma, uint4* chroma, uint32_t kw0, uint32_t kw1,
-                                         uint32_t kw2, uint32_t bias, int32_t mid)
+                                         uint32_t kw2, uint32_t bias, int32_t mid, uint32_t masked)
 {
-  using G = Geo420<R, T>;
+  using G = Geo420<R, T, TM>;
+  constexpr int MA = (G::AXM - R) % 4 == 0 ? 4 : (G::AXM - R) % 2 == 0 ? 2 : 1;
+  static_assert(!G::MASK || G::AXM - R + 4 * ((G::SW + 3) / 4) <= G::BWM, "mask units read inside the box");
   constexpr int NU = (G::SW + 3) / 4;                       // four-sample units per row; the last may hold two
   static_assert(G::AX - R + 4 * NU <= G::BWL, "units read inside the box");
   constexpr int LA = (G::AX - R) % 4 == 0 ? 4 : (G::AX - R) % 2 == 0 ? 2 : 1;
@@ -274,6 +315,13 @@ __device__ __forceinline__ void stage420(const unsigned char* raw, uint4* luma, 
       load4<T, LA>(reinterpret_cast<const T*>(raw + rowofs) + (G::AX - R) + 4 * c, v);
       #pragma unroll
       for(int k = 0; k < 4; k++) { v[k] -= (uint32_t)mid; q[k] = v[k] * v[k] * kw0; }
+      if constexpr(G::MASK)
+      {
+        uint32_t m[4];
+        load4<TM, MA>(reinterpret_cast<const TM*>(raw + G::OFFM) + (row >= G::SH ? row - G::SH : row) * G::BWM + (G::AXM - R) + 4 * c, m);
+        #pragma unroll
+        for(int k = 0; k < 4; k++) { if(m[k] == 0u) { v[k] = 0u; q[k] = masked; } }
+      }
       uint4* d = luma + row * G::LPP + c;
       d[0] = make_uint4(v[0], q[0], v[1], q[1]);
       d[G::HALF] = make_uint4(v[2], q[2], v[3], q[3]);
@@ -566,14 +614,60 @@ __device__ __forceinline__ void epilogue420(const CpsArgs& a, const unsigned cha
   }
 }
 
+// Epilogue of a masked search: squared differences weighted by the test pixels' mask values, summed per row in
+// 64 bits. A row's four terms are below 2^40 (differences below 2^13, mask values below 2^14); over the
+// warp the parts from bit 13 up (< 2^27 each) and the low 13 bits are summed in 32 bits.
+template <int R, typename T, typename TM>
+__device__ __forceinline__ void epilogue420_masked(const CpsArgs& a, const unsigned char* ref, const TM* mask, const uint32_t* off, uint32_t base,
+                                                   const uint32_t ty[16], const uint32_t tu[4], const uint32_t tv[4],
+                                                   const uint32_t idx[16], int dir, int xb, int yb, int g0, int g1, int g2)
+{
+  using G = Geo420<R, T, TM>;
+  const int lane = threadIdx.x & 31;
+  // the mask mode's labels: rows 0 hold the search of In1 in In0
+  unsigned long long* rows = a.rows64 + (size_t)(dir ^ 1) * a.H * 3;
+  uint32_t hi = 0, lo = 0;
+  #pragma unroll
+  for(int i = 0; i < 4; i++)
+  {
+    uint64_t rs[3] = { 0, 0, 0 };
+    uint32_t m[4];
+    load4<TM, 4>(mask + i * G::BWM, m);
+    #pragma unroll
+    for(int j = 0; j < 4; j++)
+    {
+      const int p = 4 * i + j, b = (i >> 1) * 2 + (j >> 1);
+      const uint32_t w = off[(2 * (i & 1) + (j & 1)) * 128 + idx[p]] + base;
+      const unsigned char* pl = ref + (w & 0xffffu);
+      const unsigned char* pc = ref + (w >> 16);
+      const int co = (i >> 1) * G::PCB + (j >> 1) * G::ESZ;
+      const uint32_t d0 = ty[p] + (uint32_t)g0 - *reinterpret_cast<const T*>(pl + i * G::PLB + j * G::ESZ);
+      const uint32_t d1 = tu[b] + (uint32_t)g1 - *reinterpret_cast<const T*>(pc + G::OFFU + co);
+      const uint32_t d2 = tv[b] + (uint32_t)g2 - *reinterpret_cast<const T*>(pc + G::OFFV + co);
+      const uint32_t mv = xb + j < a.W ? m[j] : 0u;
+      rs[0] += (uint64_t)(d0 * d0) * mv;
+      rs[1] += (uint64_t)(d1 * d1) * mv;
+      rs[2] += (uint64_t)(d2 * d2) * mv;
+    }
+    #pragma unroll
+    for(int c = 0; c < 3; c++)
+    {
+      const uint32_t h = __reduce_add_sync(kFull, (uint32_t)(rs[c] >> 13)), l = __reduce_add_sync(kFull, (uint32_t)rs[c] & 0x1fffu);
+      if(lane == 3 * i + c) { hi = h; lo = l; }
+    }
+  }
+  const uint64_t sum = ((uint64_t)hi << 13) + lo;
+  if(lane < 12 && yb + lane / 3 < a.H && sum != 0) { atomicAdd(rows + (size_t)yb * 3 + lane, (unsigned long long)sum); }
+}
+
 // Persistent tile loop over the work list (npairs > 0: pair p owns tiles [prefix[p], prefix[p + 1]) of
 // descs) or over the tiles of the one pair in `one`.
-template <int R, typename T>
-__global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid_constant__ CpsKernelArgs one,
+template <int R, typename T, typename TM>
+__global__ void __launch_bounds__(256, Geo420<R, T, TM>::CTAS) k_cps420(const __grid_constant__ CpsKernelArgs one,
                                                                 const CpsKernelArgs* __restrict__ descs,
                                                                 const int32_t* __restrict__ prefix, int npairs, int ntiles)
 {
-  using G = Geo420<R, T>;
+  using G = Geo420<R, T, TM>;
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   unsigned char* raw = smem_dyn + ((128u - (smem_u32(smem_dyn) & 127u)) & 127u);   // TMA boxes: 128-byte aligned
   uint4* luma = reinterpret_cast<uint4*>(raw + G::STAGES * G::STAGE);
@@ -603,7 +697,7 @@ __global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid
   if(t < ntiles && threadIdx.x == 0)
   {
     const Pair420 L = locate(next, t);
-    if(L.k->g.use_tma) { issue_tile420<R, T>(*L.k, npairs != 0, raw, bar, L.tile); }
+    if(L.k->g.use_tma) { issue_tile420<R, T, TM>(*L.k, npairs != 0, raw, bar, L.tile); }
   }
   // the next tile's copies, once every warp is done with the raw stage they go to
   auto issue_next = [&](int tn, uint32_t to) {
@@ -614,7 +708,7 @@ __global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid
       if(N.k->g.use_tma)
       {
         fence_proxy_async();
-        issue_tile420<R, T>(*N.k, next.p != last, raw + to * G::STAGE, bar + to, N.tile);
+        issue_tile420<R, T, TM>(*N.k, next.p != last, raw + to * G::STAGE, bar + to, N.tile);
       }
     }
   };
@@ -654,13 +748,13 @@ __global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid
     const int ntx = L.k->g.ntx;
     const int tyi = L.tile / ntx, txi = L.tile - tyi * ntx;
     const int x0 = txi * G::TW, y0 = tyi * G::TH;
-    if(!tma) { load_plain420<R, T>(a, box, x0, y0); __syncthreads(); }
+    if(!tma) { load_plain420<R, T, TM>(a, box, x0, y0); __syncthreads(); }
     const bool clip = a.clip < (sizeof(T) == 1 ? 0xffu : 0xffffu);
     const bool border = x0 < R || y0 < R || x0 + G::TW + R > a.W || y0 + G::TH + R > a.H;
-    if(clip || border) { complete_halo<R, T>(a, box, x0, y0, clip, border); }
+    if(clip || border) { complete_halo<R, T, TM>(a, box, x0, y0, clip, border); }
     const uint32_t kw0 = G::K * (uint32_t)a.wi[0], kw1 = G::K * (uint32_t)a.wi[1], kw2 = G::K * (uint32_t)a.wi[2];
     const int32_t mid = a.key_mid;
-    stage420<R, T>(box, luma, chroma, kw0, kw1, kw2, G::K * a.key_bias, mid);
+    stage420<R, T, TM>(box, luma, chroma, kw0, kw1, kw2, G::K * a.key_bias, mid, a.key_masked);
     __syncthreads();
     if(G::STAGES == 2) { issue_next(t + (int)gridDim.x, stage ^ 1u); }
     // dir 0 (R2T): test = In0 + GCD searched in In1 -> rows[0], SCP1 = clip(In1[best] - GCD)
@@ -671,7 +765,7 @@ __global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid
     const unsigned char* ref = box + (dir ^ 1) * G::PIC;
     uint32_t idx[16];
     const int lofs = 4 * by * G::BWL + (G::AX - R) + 4 * lane, cofs = 2 * by * G::BWC + (G::AX - G::CR0) + 2 * lane;
-    if((s_gcd[3] & 4) == 0)
+    if(G::MASK || (s_gcd[3] & 4) == 0)
     {
       uint32_t c0[16], c1[4], c2[4], ty[16], tu[4], tv[4];
       load_test420<R, T>(tst, by, lane, 0, ty, tu, tv);
@@ -704,6 +798,13 @@ __global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid
     load_test420<R, T>(tst, by, lane, zero, ty, tu, tv);
     const uint32_t base = (uint32_t)(lofs * G::ESZ) | ((uint32_t)(cofs * G::ESZ) << 16);
     const int xb = x0 + 4 * lane, yb = y0 + 4 * by;
+    if constexpr(G::MASK)
+    {
+      epilogue420_masked<R, T, TM>(a, ref, reinterpret_cast<const TM*>(box + G::OFFM) + (4 * by + R) * G::BWM + G::AXM + 4 * lane, s_off, base, ty, tu,
+                                   tv, idx, dir, xb, yb, g0, g1, g2);
+    }
+    else
+    {
     const int sel = ((x0 + G::TW > a.W || y0 + G::TH > a.H) ? 4 : 0) | (a.mom[dir].p != nullptr ? 2 : 0) |
                     ((dir ? a.scp0 : a.scp1) != nullptr ? 1 : 0);
     switch(sel)
@@ -716,6 +817,7 @@ __global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid
     case 5: epilogue420<R, T, true, false, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
     default: epilogue420<R, T, true, true, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;   // 3, 7
     }
+    }
     if(G::STAGES == 1)
     {
       __syncthreads();
@@ -725,51 +827,47 @@ __global__ void __launch_bounds__(256, Geo420<R, T>::CTAS) k_cps420(const __grid
 }
 
 // ---- host -------------------------------------------------------------------------------------
-// Calls f(Geo420<R, T>) for the runtime (R, sample size); false when there is no such form.
-template <typename F>
-bool with_geo(int R, int esz, F&& f)
+// Calls f(Geo420<R, T, TM>) for the runtime (R, sample size, mask sample size; 0 = no mask); false when there
+// is no such form.
+template <typename T, typename TM, typename F>
+bool with_geo_r(int R, F&& f)
 {
-  switch(R * 4 + esz)
+  switch(R)
   {
-  case 1 * 4 + 1: f(Geo420<1, uint8_t>{}); return true;
-  case 2 * 4 + 1: f(Geo420<2, uint8_t>{}); return true;
-  case 3 * 4 + 1: f(Geo420<3, uint8_t>{}); return true;
-  case 4 * 4 + 1: f(Geo420<4, uint8_t>{}); return true;
-  case 5 * 4 + 1: f(Geo420<5, uint8_t>{}); return true;
-  case 1 * 4 + 2: f(Geo420<1, uint16_t>{}); return true;
-  case 2 * 4 + 2: f(Geo420<2, uint16_t>{}); return true;
-  case 3 * 4 + 2: f(Geo420<3, uint16_t>{}); return true;
-  case 4 * 4 + 2: f(Geo420<4, uint16_t>{}); return true;
-  case 5 * 4 + 2: f(Geo420<5, uint16_t>{}); return true;
+  case 1: f(Geo420<1, T, TM>{}); return true;
+  case 2: f(Geo420<2, T, TM>{}); return true;
+  case 3: f(Geo420<3, T, TM>{}); return true;
+  case 4: f(Geo420<4, T, TM>{}); return true;
+  case 5: f(Geo420<5, T, TM>{}); return true;
+  default: return false;
+  }
+}
+template <typename F>
+bool with_geo(int R, int esz, int mesz, F&& f)
+{
+  switch(esz * 4 + mesz)
+  {
+  case 1 * 4 + 0: return with_geo_r<uint8_t, NoMask>(R, f);
+  case 1 * 4 + 1: return with_geo_r<uint8_t, uint8_t>(R, f);
+  case 1 * 4 + 2: return with_geo_r<uint8_t, uint16_t>(R, f);
+  case 2 * 4 + 0: return with_geo_r<uint16_t, NoMask>(R, f);
+  case 2 * 4 + 1: return with_geo_r<uint16_t, uint8_t>(R, f);
+  case 2 * 4 + 2: return with_geo_r<uint16_t, uint16_t>(R, f);
   default: return false;
   }
 }
 
-template <int R, typename T>
-cudaError_t launch420(const CpsKernelArgs* one, const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, cudaStream_t s)
+template <int R, typename T, typename TM>
+cudaError_t launch420(Geo420<R, T, TM>, const CpsKernelArgs* one, const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, cudaStream_t s)
 {
-  using G = Geo420<R, T>;
+  using G = Geo420<R, T, TM>;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if(e == cudaSuccess) { e = configure_once(k_cps420<R, T>, dev); }
+  if(e == cudaSuccess) { e = configure_once(k_cps420<R, T, TM>, dev); }
   if(e != cudaSuccess) { return e; }
   static const CpsKernelArgs none{};
-  k_cps420<R, T><<<grid_for(k_cps420<R, T>, G::NT, G::SMEM, ntiles, dev), G::NT, G::SMEM, s>>>(one ? *one : none, d, prefix, npairs, ntiles);
+  k_cps420<R, T, TM><<<grid_for(k_cps420<R, T, TM>, G::NT, G::SMEM, ntiles, dev), G::NT, G::SMEM, s>>>(one ? *one : none, d, prefix, npairs, ntiles);
   return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch420_r(int R, const CpsKernelArgs* one, const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, cudaStream_t s)
-{
-  switch(R)
-  {
-  case 1: return launch420<1, T>(one, d, prefix, npairs, ntiles, s);
-  case 2: return launch420<2, T>(one, d, prefix, npairs, ntiles, s);
-  case 3: return launch420<3, T>(one, d, prefix, npairs, ntiles, s);
-  case 4: return launch420<4, T>(one, d, prefix, npairs, ntiles, s);
-  case 5: return launch420<5, T>(one, d, prefix, npairs, ntiles, s);
-  default: return cudaErrorInvalidValue;
-  }
 }
 
 }  // namespace
@@ -779,7 +877,7 @@ bool cps420_fits(int R, int esz)
   int dev = 0;
   if(cudaGetDevice(&dev) != cudaSuccess) { return false; }
   bool fits = false;
-  with_geo(R, esz, [&](auto g) { using G = decltype(g); fits = (size_t)G::SMEM + 4096 <= (size_t)dev_info(dev).smem_optin; });
+  with_geo(R, esz, 0, [&](auto g) { using G = decltype(g); fits = (size_t)G::SMEM + 4096 <= (size_t)dev_info(dev).smem_optin; });
   return fits;
 }
 
@@ -790,8 +888,9 @@ cudaError_t cps420_describe(CpsKernelArgs& k, int R, int esz, CpsPairPlan* plan)
 {
   k.g.ntx = (k.a.W + 127) / 128;
   k.g.ntiles = cps420_tiles(k.a.W, k.a.H);
+  if(k.a.mask) { cps_masked_key(R, k.a.maxv, k.a.wi, k.a.gmax, &k.a.key_masked); }
   cps_shared_key(R, k.a.maxv, k.a.wi, k.a.gmax, &k.a.key_bias, &k.a.key_mid);
-  const bool known = with_geo(R, esz, [&](auto g) {
+  const bool known = with_geo(R, esz, k.a.mask ? k.a.mask_esz : 0, [&](auto g) {
     using G = decltype(g);
     bool tma = true;
     for(int f = 0; f < 2; f++)
@@ -801,6 +900,7 @@ cudaError_t cps420_describe(CpsKernelArgs& k, int R, int esz, CpsPairPlan* plan)
             cps_encode_plane(&k.map[f][1], im.p[1], k.a.W >> 1, k.a.H >> 1, im.pitch[1], esz, G::BWC, G::BHC) &&
             cps_encode_plane(&k.map[f][2], im.p[2], k.a.W >> 1, k.a.H >> 1, im.pitch[2], esz, G::BWC, G::BHC);
     }
+    if(G::MASK) { tma = tma && cps_encode_plane(&k.mask_map, k.a.mask, k.a.W, k.a.H, k.a.mask_pitch, k.a.mask_esz, G::BWM, G::BHL); }
     k.g.use_tma = tma ? 1 : 0;
     if(plan) { plan->ntiles = k.g.ntiles; plan->raw_bytes = 0; plan->smem = G::SMEM; }
   });
@@ -809,14 +909,31 @@ cudaError_t cps420_describe(CpsKernelArgs& k, int R, int esz, CpsPairPlan* plan)
 
 cudaError_t cps420_launch(const CpsKernelArgs& k, int R, int esz, cudaStream_t s)
 {
-  return esz == 1 ? launch420_r<uint8_t>(R, &k, nullptr, nullptr, 0, k.g.ntiles, s)
-                  : launch420_r<uint16_t>(R, &k, nullptr, nullptr, 0, k.g.ntiles, s);
+  cudaError_t e = cudaErrorInvalidValue;
+  with_geo(R, esz, k.a.mask ? k.a.mask_esz : 0, [&](auto g) { e = launch420(g, &k, nullptr, nullptr, 0, k.g.ntiles, s); });
+  return e;
 }
 
-cudaError_t cps420_launch_multi(const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, int R, int esz, cudaStream_t s)
+cudaError_t cps420_launch_multi(const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, int R, int esz, int mesz, cudaStream_t s)
 {
-  return esz == 1 ? launch420_r<uint8_t>(R, nullptr, d, prefix, npairs, ntiles, s)
-                  : launch420_r<uint16_t>(R, nullptr, d, prefix, npairs, ntiles, s);
+  cudaError_t e = cudaErrorInvalidValue;
+  with_geo(R, esz, mesz, [&](auto g) { e = launch420(g, nullptr, d, prefix, npairs, ntiles, s); });
+  return e;
+}
+
+cudaError_t launch_cps_masked420(const CpsArgs& a, int R, int esz, cudaStream_t s)
+{
+  CpsKernelArgs k;
+  std::memset(&k, 0, sizeof(k));
+  k.a = a;
+  k.g.status = const_cast<int32_t*>(&a.gcd_src->flags);
+  const cudaError_t e = cps420_describe(k, R, esz, nullptr);
+  return e != cudaSuccess ? e : cps420_launch(k, R, esz, s);
+}
+
+cudaError_t launch_cps_masked420_multi(const void* d_descs, const int32_t* d_prefix, int npairs, int ntiles, int R, int esz, int mesz, cudaStream_t s)
+{
+  return cps420_launch_multi(static_cast<const CpsKernelArgs*>(d_descs), d_prefix, npairs, ntiles, R, esz, mesz, s);
 }
 
 // Integer keys: with |s'| <= mid + |GCD|, |r'| <= mid, the subtracted terms are at most
@@ -825,7 +942,7 @@ bool cps_shared_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[
 {
   const int64_t m = ((int64_t)maxv + 1) / 2;
   const int D = 2 * R + 1;
-  const int64_t K = R <= 2 ? 32 : (R == 3 ? 64 : 128);
+  const int64_t K = (int64_t)1 << key_bits(R);
   long double lo = 0, hi = 0;
   for(int c = 0; c < 3; c++)
   {
@@ -838,6 +955,29 @@ bool cps_shared_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[
   if(bias) { *bias = ok ? (uint32_t)lo : 0u; }
   if(mid) { *mid = (int32_t)m; }
   return ok;
+}
+
+// Masked search: a masked sample's keys, masked + P + code, must lie above every real key and below 2^32.
+// P lies between K w_0 (mid + g_0)^2 and K (lo + hi_1 + hi_2), with lo and hi as above; the row sums need
+// differences below 2^13.
+bool cps_masked_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[3], uint32_t* masked)
+{
+  if(!cps_shared_key(R, maxv, w, gmax, nullptr, nullptr)) { return false; }
+  const int64_t m = ((int64_t)maxv + 1) / 2, D = 2 * R + 1, K = (int64_t)1 << key_bits(R), code = (3 + 2 * R) * D + 3 + 2 * R;
+  int64_t lo = 0, hi = 0, hic = 0;   // bounded by cps_shared_key
+  bool small = true;
+  for(int c = 0; c < 3; c++)
+  {
+    const int64_t g = gmax[c] < 0 ? -(int64_t)gmax[c] : gmax[c], h = (int64_t)w[c] * (m * m + 2 * (m + g) * m);
+    lo += (int64_t)w[c] * (m + g) * (m + g);
+    hi += h;
+    if(c) { hic += h; }
+    small = small && maxv + g < (1 << 13);
+  }
+  const int64_t g0 = gmax[0] < 0 ? -(int64_t)gmax[0] : gmax[0];
+  const int64_t big = K * (lo + hi) + code + 1 - K * (int64_t)w[0] * (m + g0) * (m + g0);
+  if(masked) { *masked = (uint32_t)big; }
+  return small && big + K * (lo + hic) + code < ((int64_t)1 << 32);
 }
 
 }  // namespace qmiv

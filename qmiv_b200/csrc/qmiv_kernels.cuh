@@ -52,6 +52,12 @@ struct CpsArgs
   int32_t        gmax[3];      // bound of |GCD| per component
   int32_t        key_mid;      // 4:2:0 form: mid value and key bias (set when the pair is described)
   uint32_t       key_bias;
+  // masked 4:2:0 search: luma plane of the mask (null = none), its pitch in samples and bytes per
+  // sample, the staged value of a masked sample, 64-bit row sums [2][H][3]
+  const void*    mask;
+  int32_t        mask_pitch, mask_esz;
+  uint32_t       key_masked;
+  unsigned long long* rows64;
   const PairOut* gcd_src;      // gcd + flags
   uint32_t*      rows;         // [2][H][3], zeroed, 32-bit wrap-around sums
   void*          scp0;         // In0 resampled (T2R search result), planar 3 x W*H, may be null
@@ -212,10 +218,16 @@ cudaError_t cps_describe(void* desc, const CpsArgs& a, int R, int esz, int wy, C
 cudaError_t launch_cps_multi(const void* d_descs, const int32_t* d_prefix, int npairs, int ntiles, int R, int wy,
                              int esz, uint32_t raw_cap, size_t smem, cudaStream_t s);
 
+// The masked search of 4:2:0 pictures (CpsArgs::mask set) for one pair, and for a work list of described pairs
+cudaError_t launch_cps_masked420(const CpsArgs& a, int R, int esz, cudaStream_t s);
+cudaError_t launch_cps_masked420_multi(const void* d_descs, const int32_t* d_prefix, int npairs, int ntiles, int R, int esz, int mesz, cudaStream_t s);
+
 // Exactness check of the fp32 key path for a given bit depth, weights and GCD clip range.
 bool cps_fp32_exact(int32_t maxv, const int32_t w[3], const int32_t maxdiff[3]);
 // The same for the integer keys of the 4:2:0 form (qmiv_cps420.cu), with the constants its keys use.
 bool cps_shared_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[3], uint32_t* bias, int32_t* mid);
+// ... and for its masked search.
+bool cps_masked_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[3], uint32_t* masked);
 // ... for the form a picture of these chroma shifts is searched with.
 bool cps_key_exact(int R, int sx, int sy, int32_t maxv, const int32_t w[3], const int32_t maxdiff[3]);
 // Tile form 1 is the 4:2:0 form; the others are the warps of a tile column.

@@ -14,7 +14,7 @@
 //                    are weighted by the test pixel's mask value and summed per row in uint64;
 //                    k_cps_masked_key is the same search by exact fp32 keys, both directions per
 //                    CTA, four pixels per thread, where the bit depth, weights and GCD range bound
-//                    every error
+//                    every error; 4:2:0 pictures take the integer-key search of qmiv_cps420.cu
 //   k_mask_finalize  the ordered compensated sums (xKBNS.h:36-43) of the ERP row weights and the
 //                    row totals, one CTA per chain (terms staged in shared memory, one thread sums)
 // dB values, exact-component fake values and the picture averages are formed on the host in
@@ -26,6 +26,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cstddef>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -66,7 +67,6 @@ struct MaskArgs
   const double* ws;            // [H] or null
   MaskOut*    out;
   uint32_t    kscale;          // 128, read from the parameter bank so the key stays one integer multiply-add
-  int32_t     pairs420;        // 4:2:0 with luma and mask rows on 2-sample boundaries (two-sample loads)
 };
 
 // Host-side description of one masked frame pair: its shape and parameters and what follows from them
@@ -79,6 +79,7 @@ struct MaskPlan
   size_t              mesz = 1;      // bytes per mask sample
   int32_t             maxdiff[4] = { 0, 0, 0, 0 };
   bool                key = false;   // the exact-key search applies (k_cps_masked_key)
+  bool                key420 = false;   // the 4:2:0 integer-key search applies (qmiv_cps420.cu)
   double              ws_corr = 1.0;
   std::vector<double> ws;            // [H] with ERP
 };
@@ -778,77 +779,6 @@ struct MaskKeyGeo
   static constexpr size_t kSmem = sizeof(float4) * 2 * SH * SW + sizeof(int32_t) * TH * TW;
 };
 
-// Two adjacent samples of one row (the host checked the alignment): low sample first
-__device__ __forceinline__ void ld_pair(const uint16_t* p, uint32_t& v0, uint32_t& v1)
-{
-  const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p));
-  v0 = w & 0xffffu; v1 = w >> 16;
-}
-__device__ __forceinline__ void ld_pair(const uint8_t* p, uint32_t& v0, uint32_t& v1)
-{
-  const uint32_t w = __ldg(reinterpret_cast<const unsigned short*>(p));
-  v0 = w & 0xffu; v1 = w >> 8;
-}
-
-// The key search's staging for a tile whose halo lies inside a 4:2:0 picture, R even: the staged area
-// splits into 2 x 2 blocks at even picture coordinates, each under one chroma sample, read as two-sample
-// rows of luma and mask and one sample per chroma plane; the chroma part of the key, w1 Cb^2 + w2 Cr^2,
-// is formed once per block. Under the key search's bound every partial sum of the key is an integer
-// below 2^24, so the key equals the per-sample form's whatever the order of the additions.
-template <typename T, typename TM, int R>
-__device__ __forceinline__ void stage_key420(const MaskArgs& a, float4* st0, float4* st1, int32_t* mk, int x0, int y0,
-                                             float w0, float w1, float w2)
-{
-  using G = MaskKeyGeo<R>;
-  constexpr int TW = G::TW, TH = G::TH, SW = G::SW, SH = G::SH, BW = SW / 2;
-  const bool clip_on = a.clip < (sizeof(T) == 1 ? 0xffu : 0xffffu);
-  for(int b = threadIdx.x; b < (SH / 2) * BW; b += 512)
-  {
-    const int by = b / BW, bx = b - by * BW;
-    const int ly = 2 * by, lx = 2 * bx;
-    const int ux = x0 - R + lx, uy = y0 - R + ly;             // even, the block inside the picture
-    uint32_t m[4];
-    {
-      const TM* mp = static_cast<const TM*>(a.mask) + (size_t)uy * a.mpitch + ux;
-      ld_pair(mp, m[0], m[1]);
-      ld_pair(mp + a.mpitch, m[2], m[3]);
-    }
-    const Img* im[2] = { &a.in0, &a.in1 };
-    float4* st[2] = { st0, st1 };
-    #pragma unroll
-    for(int f = 0; f < 2; f++)
-    {
-      const T* yp = static_cast<const T*>(im[f]->p[0]) + (size_t)uy * im[f]->pitch[0] + ux;
-      uint32_t v[4];
-      ld_pair(yp, v[0], v[1]);
-      ld_pair(yp + im[f]->pitch[0], v[2], v[3]);
-      uint32_t cb = __ldg(static_cast<const T*>(im[f]->p[1]) + (size_t)(uy >> 1) * im[f]->pitch[1] + (ux >> 1));
-      uint32_t cr = __ldg(static_cast<const T*>(im[f]->p[2]) + (size_t)(uy >> 1) * im[f]->pitch[2] + (ux >> 1));
-      if(clip_on)
-      {
-        cb = min(cb, a.clip); cr = min(cr, a.clip);
-        #pragma unroll
-        for(int i = 0; i < 4; i++) { v[i] = min(v[i], a.clip); }
-      }
-      const float fb = u2f_exact(cb), fr = u2f_exact(cr);
-      const float ct = fmaf(w2, fr * fr, fmaf(w1, fb * fb, kMaskBias));
-      #pragma unroll
-      for(int i = 0; i < 4; i++)
-      {
-        const float fy = u2f_exact(v[i]);
-        const int e = (ly + (i >> 1)) * SW + lx + (i & 1);
-        st[f][e] = m[i] ? make_float4(fy, fb, fr, fmaf(w0, fy * fy, ct)) : make_float4(0.f, 0.f, 0.f, kMaskedValue);
-      }
-    }
-    #pragma unroll
-    for(int i = 0; i < 4; i++)
-    {
-      const int ty = ly + (i >> 1) - R, tx = lx + (i & 1) - R;
-      if(ty >= 0 && ty < TH && tx >= 0 && tx < TW) { mk[ty * TW + tx] = (int32_t)m[i]; }
-    }
-  }
-}
-
 template <typename T, typename TM, int R>
 // kscale: 128 from a kernel parameter at a fixed offset (the key stays one multiply-add with a constant operand)
 __device__ __forceinline__ void cps_masked_key_body(const MaskArgs& a, int bx, int by, uint32_t kscale)
@@ -862,16 +792,7 @@ __device__ __forceinline__ void cps_masked_key_body(const MaskArgs& a, int bx, i
   int32_t* mk = reinterpret_cast<int32_t*>(smem + 2 * SH * SW);   // M of the tile's pixels, 0 outside the picture
   const int x0 = bx * TW, y0 = by * TH;
   const float w0 = (float)a.cws[0], w1 = (float)a.cws[1], w2 = (float)a.cws[2];
-  bool staged = false;
-  if constexpr(R % 2 == 0)
-  {
-    if(a.pairs420 && x0 >= R && y0 >= R && x0 + TW + R <= a.W && y0 + TH + R <= a.H)
-    {
-      stage_key420<T, TM, R>(a, st0, st1, mk, x0, y0, w0, w1, w2);
-      staged = true;
-    }
-  }
-  for(int e = staged ? SH * SW : threadIdx.x; e < SH * SW; e += 512)
+  for(int e = threadIdx.x; e < SH * SW; e += 512)
   {
     const int ly = e / SW, lx = e - ly * SW;
     const int ux = x0 - R + lx, uy = y0 - R + ly;
@@ -1135,7 +1056,7 @@ cudaError_t launch_masked_key(const MaskArgs& a, cudaStream_t s)
 
 // pipe: the stage timers of the calling calc (events around each stage when its context profiles)
 template <typename T, typename TM>
-cudaError_t launch_masked_t(const MaskArgs& a, int R, bool key, PairPipeline& pipe, cudaStream_t s)
+cudaError_t launch_masked_t(const MaskArgs& a, int R, bool key, const CpsArgs* c420, PairPipeline& pipe, cudaStream_t s)
 {
   int tok = pipe.prof_begin(s);
   if(mask_prepass_vec_ok(a, sizeof(T), sizeof(TM))) { k_mask_prepass420v<T, TM><<<prepass420_units<TM>(a.H), 256, 0, s>>>(a); }
@@ -1146,7 +1067,12 @@ cudaError_t launch_masked_t(const MaskArgs& a, int R, bool key, PairPipeline& pi
   pipe.prof_end(s, QMIV_STAGE_REDUCE, tok);
   tok = pipe.prof_begin(s);
   const dim3 grid((a.W + 31) / 32, (a.H + 7) / 8, 2);
-  if(key)
+  if(c420)
+  {
+    const cudaError_t e = launch_cps_masked420(*c420, R, (int)sizeof(T), s);
+    if(e != cudaSuccess) { return e; }
+  }
+  else if(key)
   {
     cudaError_t e;
     switch(R)
@@ -1233,6 +1159,10 @@ qmiv_status plan_masked(const Shape& S, const qmiv_params& prm, const qmiv_frame
   P.key = (prm.invalid_pel_action == QMIV_PEL_STOP || prm.invalid_pel_action == QMIV_PEL_CNCL) &&
           cps_fp32_exact(S.maxv, prm.cws, P.maxdiff) && ((int64_t)1 << 23) + bound <= ((int64_t)1 << 24) - 2 &&
           dmax2 < ((int64_t)1 << 24);
+  // 4:2:0 pictures whose integer keys leave room for masked samples (every one that the fp32 keys take
+  // at default weights, and 11 bits up to R = 3)
+  P.key420 = (prm.invalid_pel_action == QMIV_PEL_STOP || prm.invalid_pel_action == QMIV_PEL_CNCL) && S.sx == 1 && S.sy == 1 &&
+             cps_masked_key(prm.search_range, S.maxv, prm.cws, P.maxdiff, nullptr);
   P.ws.clear();
   P.ws_corr = 1.0;
   if(prm.erp) { ws_weights_cached(S.H, prm.lat_range_deg, P.ws, P.ws_corr); }
@@ -1269,18 +1199,25 @@ void fill_mask_args(const MaskPlan& P, const Img& a0, const Img& a1, uint64_t* r
   a.ws = P.prm.erp ? ws : nullptr;
   a.out = out;
   a.kscale = 128u;
-  auto al = [](const void* q, size_t n) { return (reinterpret_cast<uintptr_t>(q) % n) == 0; };
-  bool ok = a.mask != nullptr && a.mpitch % 2 == 0 && al(a.mask, 2 * P.mesz);
-  for(const Img* im : { &a.in0, &a.in1 })
-  {
-    ok = ok && im->sx[0] == 0 && im->sy[0] == 0 && im->pitch[0] % 2 == 0 && al(im->p[0], 2 * S.esz);
-    for(int c = 1; c < 3; c++) { ok = ok && im->sx[c] == 1 && im->sy[c] == 1; }
-  }
-  a.pairs420 = ok ? 1 : 0;
+}
+
+// Arguments of the 4:2:0 integer-key search. It reads the GCD and the flags of a result block through
+// PairOut, whose first members are MaskOut's.
+static CpsArgs mask_cps_args(const MaskPlan& P, const MaskArgs& a)
+{
+  static_assert(offsetof(PairOut, gcd) == offsetof(MaskOut, gcd) && offsetof(PairOut, flags) == offsetof(MaskOut, flags), "shared first members");
+  CpsArgs c{};
+  c.in0 = a.in0; c.in1 = a.in1; c.W = a.W; c.H = a.H; c.maxv = a.maxv; c.clip = a.clip;
+  for(int k = 0; k < 3; k++) { c.wi[k] = a.cws[k]; c.wf[k] = (float)a.cws[k]; c.gmax[k] = a.maxdiff[k]; }
+  c.gcd_src = reinterpret_cast<const PairOut*>(a.out);
+  c.mask = a.mask; c.mask_pitch = a.mpitch; c.mask_esz = (int32_t)P.mesz;
+  c.rows64 = reinterpret_cast<unsigned long long*>(a.row_cps);
+  return c;
 }
 
 qmiv_status masked_status(const MaskOut& o, const MaskPlan& P)
 {
+  if(o.flags & 8) { return fail(QMIV_ERR_TIMEOUT, "a CPS tile load did not complete within its wait bound"); }
   if(P.prm.invalid_pel_action == QMIV_PEL_STOP && (o.flags & 3))
   {
     return fail(QMIV_ERR_INVALID_PIXEL, "input frame contains samples above the bit depth's maximum");
@@ -1371,9 +1308,17 @@ qmiv_status MaskedPipeline::run(qmiv_calc_s* calc, const qmiv_frame* in0, const 
   QMIV_CUDA(cudaMemsetAsync(out_.p, 0, sizeof(MaskOut), s));
   QMIV_CUDA(cudaMemsetAsync(a.row_cps, 0, (size_t)6 * S.H * sizeof(uint64_t), s));
   const int R = P.prm.search_range;
+  const CpsArgs ca = mask_cps_args(P, a);
+  const CpsArgs* c420 = P.key420 ? &ca : nullptr;
   cudaError_t e;
-  if(S.esz == 1) { e = P.mesz == 1 ? launch_masked_t<uint8_t, uint8_t>(a, R, P.key, pipe, s) : launch_masked_t<uint8_t, uint16_t>(a, R, P.key, pipe, s); }
-  else { e = P.mesz == 1 ? launch_masked_t<uint16_t, uint8_t>(a, R, P.key, pipe, s) : launch_masked_t<uint16_t, uint16_t>(a, R, P.key, pipe, s); }
+  if(S.esz == 1)
+  {
+    e = P.mesz == 1 ? launch_masked_t<uint8_t, uint8_t>(a, R, P.key, c420, pipe, s) : launch_masked_t<uint8_t, uint16_t>(a, R, P.key, c420, pipe, s);
+  }
+  else
+  {
+    e = P.mesz == 1 ? launch_masked_t<uint16_t, uint8_t>(a, R, P.key, c420, pipe, s) : launch_masked_t<uint16_t, uint16_t>(a, R, P.key, c420, pipe, s);
+  }
   if(e != cudaSuccess) { return cuda_fail(e, "masked launches"); }
   const int tok = pipe.prof_begin(s);
   QMIV_CUDA(cudaMemcpyAsync(h_out_, out_.p, sizeof(MaskOut), cudaMemcpyDeviceToHost, s));
@@ -1457,9 +1402,9 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
                              int32_t* num_non_masked)
 {
   std::vector<MaskPlan> P(n);
-  size_t off_out = 0, off_rows = malign(sizeof(MaskOut) * n), cur = 0;
+  size_t off_out = 0, cur = malign(sizeof(MaskOut) * n);
   std::vector<size_t> o_rows(n), o_stage(n), o_mstage(n);
-  cur = off_rows;
+  int n420 = 0;
   for(int i = 0; i < n; i++)
   {
     const qmiv_pair_desc& d = pairs[i];
@@ -1474,6 +1419,13 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
     QMIV_TRY(validate_params(prm));
     QMIV_TRY(plan_masked(S, prm, &masks[i], mask_bitdepths[i], P[i]));
     o_rows[i] = cur; cur += malign(sizeof(uint64_t) * 9 * S.H);
+    n420 += P[i].key420 ? 1 : 0;
+  }
+  const size_t zero_bytes = cur;                            // results and row sums start at zero
+  for(int i = 0; i < n; i++)
+  {
+    const qmiv_pair_desc& d = pairs[i];
+    const Shape& S = P[i].S;
     const bool host = d.in0.mem == QMIV_MEM_HOST || d.in1.mem == QMIV_MEM_HOST;
     o_stage[i] = cur; cur += host ? malign(2 * S.staged_frame_bytes()) : 0;
     o_mstage[i] = cur; cur += masks[i].mem == QMIV_MEM_HOST ? malign((size_t)S.W * P[i].mesz * S.H) : 0;
@@ -1481,9 +1433,10 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
   // groups: prepass by (sample sizes, prepass form), search by (sample sizes, R, search form)
   std::map<std::tuple<int, int, int>, GroupInfo> pre;
   std::map<std::tuple<int, int, int, int>, GroupInfo> srch;
-  const size_t total = cur;
-  QMIV_TRY(arena_.ensure(ctx, total));
-  const size_t hbytes = sizeof(MaskOut) * n;
+  // work-list descriptors of the 4:2:0 searches, then the tile prefixes of their groups (at most one per pair)
+  const size_t o_desc = malign(cur), desc_bytes = malign(cps_desc_bytes() * n420), prefix_bytes = sizeof(int32_t) * 2 * n420;
+  QMIV_TRY(arena_.ensure(ctx, o_desc + desc_bytes + prefix_bytes));
+  const size_t h_desc = malign(sizeof(MaskOut) * n), hbytes = h_desc + desc_bytes + prefix_bytes;
   if(h_bytes_ < hbytes)
   {
     if(h_) { cudaFreeHost(h_); h_ = nullptr; h_bytes_ = 0; }
@@ -1493,7 +1446,7 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
   char* dbase = arena_.as<char>();
   std::vector<MaskArgs> hargs(n);
   MaskOut* hout = static_cast<MaskOut*>(h_);
-  QMIV_CUDA(cudaMemsetAsync(dbase, 0, total, s));          // results and row sums start at zero
+  QMIV_CUDA(cudaMemsetAsync(dbase, 0, zero_bytes, s));
   for(int i = 0; i < n; i++)
   {
     const MaskPlan& p = P[i];
@@ -1522,7 +1475,35 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
     const int t = (int)S.esz, tm = (int)p.mesz;
     const int form = mask_prepass_vec_ok(a, S.esz, p.mesz) ? 1 : 0;
     pre[std::make_tuple(t, tm, form)].pairs.push_back(i);
-    srch[std::make_tuple(t, tm, p.prm.search_range, (int)p.key)].pairs.push_back(i);
+    srch[std::make_tuple(t, tm, p.prm.search_range, p.key420 ? 2 : (int)p.key)].pairs.push_back(i);
+  }
+  // 4:2:0 searches: descriptors and tile prefixes of every group, one copy for all
+  struct List { const void* desc; const int32_t* prefix; int tiles; };
+  std::map<std::tuple<int, int, int, int>, List> lists;
+  if(n420 > 0)
+  {
+    char* hd = static_cast<char*>(h_) + h_desc;
+    int32_t* hp = reinterpret_cast<int32_t*>(hd + desc_bytes);
+    size_t di = 0, pi = 0;
+    for(const auto& g : srch)
+    {
+      if(std::get<3>(g.first) != 2) { continue; }
+      List& L = lists[g.first];
+      L.desc = dbase + o_desc + di * cps_desc_bytes();
+      L.prefix = reinterpret_cast<const int32_t*>(dbase + o_desc + desc_bytes) + pi;
+      L.tiles = 0;
+      for(int32_t i : g.second.pairs)
+      {
+        CpsPairPlan plan{};
+        const cudaError_t e = cps_describe(hd + di * cps_desc_bytes(), mask_cps_args(P[i], hargs[i]), std::get<2>(g.first), std::get<0>(g.first), kCpsForm420, &plan);
+        if(e != cudaSuccess) { return cuda_fail(e, "masked search descriptor"); }
+        hp[pi++] = L.tiles;
+        L.tiles += plan.ntiles;
+        di++;
+      }
+      hp[pi++] = L.tiles;
+    }
+    QMIV_CUDA(cudaMemcpyAsync(dbase + o_desc, hd, desc_bytes + prefix_bytes, cudaMemcpyHostToDevice, s));
   }
   // launches over chunks of up to kPackPairs pairs, each chunk's arguments in the launch's parameters
   std::vector<int32_t> all(n);
@@ -1562,6 +1543,13 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
   {
     const int t = std::get<0>(g.first), tm = std::get<1>(g.first), R = std::get<2>(g.first);
     const bool key = std::get<3>(g.first) != 0;
+    if(std::get<3>(g.first) == 2)
+    {
+      const List& L = lists[g.first];
+      const cudaError_t e = launch_cps_masked420_multi(L.desc, L.prefix, (int)g.second.pairs.size(), L.tiles, R, t, tm, s);
+      if(e != cudaSuccess) { return cuda_fail(e, "masked search launch"); }
+      continue;
+    }
     for(size_t f = 0; f < g.second.pairs.size(); f += kPackPairs)
     {
       const int cnt = pack(g.second.pairs, f);

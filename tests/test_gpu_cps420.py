@@ -68,3 +68,27 @@ def test_planes_without_tma(bd, qctx, oracle_lib):
         return tuple(out)
     f0, f1 = synth.make_pair(262, 50, bd, seed=11)
     _check(qctx, oracle_lib, (262, 50, bd, 2), f0, f1, dev)
+
+
+@pytest.mark.parametrize("size", SIZES[1:])
+@pytest.mark.parametrize("bd,mbd,R", [(8, 8, 2), (10, 8, 2), (10, 10, 1), (10, 14, 5), (11, 8, 3), (11, 12, 4), (12, 8, 2)])
+def test_masked_tiles(size, bd, mbd, R, qctx, oracle_lib):
+    """The masked search: single kept samples, weights over the mask's range, extreme picture samples, the
+    depths at which a masked sample's key still fits and those past it; aligned and unaligned device planes."""
+    import torch
+    W, H = size
+    rng = np.random.default_rng(bd * 100 + mbd + R)
+    top, dt, mdt = (1 << bd) - 1, np.uint8 if bd == 8 else np.uint16, np.uint8 if mbd == 8 else np.uint16
+    f = [tuple(np.where(rng.random((H >> s, W >> s)) < 0.5, rng.integers(0, top + 1, (H >> s, W >> s)),
+                        rng.choice([0, top], (H >> s, W >> s))).astype(dt) for s in (0, 1, 1)) for _ in range(2)]
+    m = np.where(rng.random((H, W)) < 0.3, rng.integers(1, 1 << mbd, (H, W)), 0).astype(mdt)
+    m[0, 0] = m[H - 1, W - 1] = (1 << mbd) - 1
+    exp, nnm = oracle_lib.compute_pair_masked(oracle.make_params(W, H, bd, 420, search_range=R, erp=True), *f, m, mbd)
+    def dev(a, extra):
+        t = torch.zeros(a.shape[0], a.shape[1] + extra, dtype=torch.uint8 if a.dtype == np.uint8 else torch.uint16, device="cuda")
+        t[:, :a.shape[1]] = torch.from_numpy(np.ascontiguousarray(a)).cuda()
+        return t[:, :a.shape[1]]
+    with qmiv_b200.Calc(qctx, W, H, bd, 420, search_range=R, erp=True) as calc:
+        for planes in ((*f, m), (*[tuple(dev(p, 5) for p in x) for x in f], dev(m, 3)), (*[tuple(dev(p, -p.shape[1] % 16) for p in x) for x in f], dev(m, -W % 16))):
+            got, n = calc.compute_masked(*planes, mbd)
+            assert n == nnm and {k: got[k] for k in exp} == exp
