@@ -18,6 +18,8 @@ objects exposing __cuda_array_interface__ (device memory), uint8 for bit depth <
 from __future__ import annotations
 
 import ctypes
+import struct
+import sys
 from typing import Iterable, Sequence
 
 import numpy as np
@@ -77,8 +79,26 @@ def make_params(search_range=2, cws=(4, 1, 1, 0), cwa=(4, 1, 1, 0), unc=(0.01, 0
     return p
 
 
+_tensor_types = None   # (torch.Tensor, torch.uint8, torch.uint16) once torch has been imported by the caller
+
+
 def _plane_info(plane):
     """(pointer, pitch in bytes, mem kind, keep-alive object) of one plane."""
+    # CUDA tensors of samples directly: their __cuda_array_interface__ costs about 4 us a plane, which at six
+    # planes a pair was a tenth to a third of a batched call
+    global _tensor_types
+    if _tensor_types is None and hasattr(sys.modules.get("torch"), "uint16"):
+        torch = sys.modules["torch"]
+        _tensor_types = (torch.Tensor, torch.uint8, torch.uint16)
+    if _tensor_types is not None and type(plane) is _tensor_types[0] and plane.is_cuda:
+        dtype = plane.dtype
+        itemsize = 1 if dtype is _tensor_types[1] else 2 if dtype is _tensor_types[2] else 0
+        if itemsize and plane.dim() == 2:
+            if plane.is_contiguous():
+                return plane.data_ptr(), plane.size(1) * itemsize, _lib.MEM_DEVICE, plane
+            if plane.stride(1) != 1:
+                raise ValueError("device plane rows must be contiguous")
+            return plane.data_ptr(), plane.stride(0) * itemsize, _lib.MEM_DEVICE, plane
     cai = getattr(plane, "__cuda_array_interface__", None)
     if cai is not None:
         shape, strides = cai["shape"], cai.get("strides")
@@ -133,21 +153,25 @@ def frame_from_raw(buffer, width: int, height: int, bitdepth: int, chroma_format
     return tuple(planes)
 
 
-def make_frame(planes: Sequence) -> tuple[_lib.QmivFrame, list]:
+_FRAME = struct.Struct("@3P3qi4x")          # qmiv_frame
+assert _FRAME.size == ctypes.sizeof(_lib.QmivFrame)
+
+
+def _pack_frame(buffer, offset, planes, keep):
+    """Writes one frame's qmiv_frame into buffer and adds its keep-alive objects to keep."""
     if len(planes) != 3:
         raise ValueError("a frame has three planes (Y, Cb, Cr)")
-    f = _lib.QmivFrame()
-    keep, mems = [], set()
-    for c, pl in enumerate(planes):
-        ptr, pitch, mem, k = _plane_info(pl)
-        f.plane[c] = ptr
-        f.pitch[c] = pitch
-        mems.add(mem)
-        keep.append(k)
-    if len(mems) != 1:
+    (p0, s0, m0, k0), (p1, s1, m1, k1), (p2, s2, m2, k2) = map(_plane_info, planes)
+    if m0 != m1 or m0 != m2:
         raise ValueError("all planes of a frame must live in the same memory")
-    f.mem = mems.pop()
-    return f, keep
+    _FRAME.pack_into(buffer, offset, p0, p1, p2, s0, s1, s2, m0)
+    keep += (k0, k1, k2)
+
+
+def make_frame(planes: Sequence) -> tuple[_lib.QmivFrame, list]:
+    buffer, keep = bytearray(_FRAME.size), []
+    _pack_frame(buffer, 0, planes, keep)
+    return _lib.QmivFrame.from_buffer(buffer), keep
 
 
 class Context:
@@ -338,14 +362,13 @@ class Batch:
 
     @staticmethod
     def _descs(pairs):
-        descs = (_lib.QmivPairDesc * max(1, len(pairs)))()
-        keep = []
+        size = ctypes.sizeof(_lib.QmivPairDesc)
+        buffer, keep = bytearray(size * max(1, len(pairs))), []
+        descs = (_lib.QmivPairDesc * max(1, len(pairs))).from_buffer(buffer)
         for i, p in enumerate(pairs):
-            f0, k0 = make_frame(p["frame0"])
-            f1, k1 = make_frame(p["frame1"])
-            keep += [k0, k1]
+            _pack_frame(buffer, i * size, p["frame0"], keep)
+            _pack_frame(buffer, i * size + _FRAME.size, p["frame1"], keep)
             d = descs[i]
-            d.in0, d.in1 = f0, f1
             d.width, d.height, d.bitdepth = p["width"], p["height"], p["bitdepth"]
             d.chroma_format = p.get("chroma_format", 420)
             d.search_range = p.get("search_range", 2)
@@ -368,9 +391,11 @@ class Batch:
         pairs = list(pairs)
         n = len(pairs)
         descs, keep = self._descs(pairs)
-        fm = (_lib.QmivFrame * max(1, n))()
+        mbuf = bytearray(_FRAME.size * max(1, n))
+        fm = (_lib.QmivFrame * max(1, n)).from_buffer(mbuf)
         for i, m in enumerate(masks):
-            fm[i], k = make_frame((m, m, m))
+            ptr, pitch, mem, k = _plane_info(m)
+            _FRAME.pack_into(mbuf, i * _FRAME.size, ptr, ptr, ptr, pitch, pitch, pitch, mem)
             keep.append(k)
         bds = (ctypes.c_int32 * max(1, n))(*mask_bitdepths)
         out = (_lib.QmivResult * max(1, n))()

@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG, "libqmiv_b200.so")
@@ -58,11 +59,24 @@ class QmivResult(ctypes.Structure):
     ]
 
     def as_dict(self):
-        d = {}
-        for name, _ in self._fields_:
-            v = getattr(self, name)
-            d[name] = list(v) if hasattr(v, "__len__") else v
-        return d
+        v = _RESULT.unpack_from(self)
+        return {name: list(v[first:first + n]) if n else v[first] for name, first, n in _RESULT_FIELDS}
+
+
+def _result_layout():
+    """One struct format for all fields of a result, and each field's name, first value and length (0: a number)."""
+    fmt, fields, first = "@", [], 0
+    codes = {ctypes.c_int32: "i", ctypes.c_uint64: "Q", ctypes.c_double: "d"}
+    for name, t in QmivResult._fields_:
+        n = getattr(t, "_length_", 0)
+        fmt += f"{max(n, 1)}{codes[t._type_ if n else t]}"
+        fields.append((name, first, n))
+        first += max(n, 1)
+    return struct.Struct(fmt), fields
+
+
+_RESULT, _RESULT_FIELDS = _result_layout()
+assert _RESULT.size == ctypes.sizeof(QmivResult)
 
 
 class QmivPairDesc(ctypes.Structure):

@@ -265,3 +265,20 @@ def test_shared_chroma_keys_order_like_int32_errors(bd, w, R):
         key = u(-2 * K * wi[0] * sc[:, None, 0]) * u(rc[..., 0]) + t
         assert np.array_equal(np.argmin(key, axis=1), best)
         assert np.array_equal((key.min(axis=1) - u(i * D + j)) & np.uint32(K - 1), best)
+
+
+def test_result_and_frame_packing_match_the_ctypes_fields():
+    """as_dict's one unpack equals reading every field; a packed frame holds its planes' pointers and pitches."""
+    import ctypes
+    import qmiv_b200
+    from qmiv_b200 import _lib
+    rng = np.random.default_rng(3)
+    r = _lib.QmivResult.from_buffer_copy(rng.bytes(ctypes.sizeof(_lib.QmivResult)))
+    for name, first in ((n, getattr(r, n)) for n, _ in r._fields_):
+        want = list(first) if hasattr(first, "__len__") else first
+        assert repr(r.as_dict()[name]) == repr(want)
+    base = np.zeros((12, 40), np.uint16)
+    planes = (base[:, :32], base[:6, 8:24], base[6:, 8:24])
+    f, keep = qmiv_b200.make_frame(planes)
+    assert [f.plane[c] for c in range(3)] == [p.ctypes.data for p in planes] and list(f.pitch) == [80] * 3
+    assert f.mem == _lib.MEM_HOST and all(k is p for k, p in zip(keep, planes))
