@@ -189,13 +189,8 @@ qmiv_status PairPipeline::prepare(uint32_t mask, bool want_scp, bool host_frames
   const bool need_ms = mask & (QMIV_MSSSIM | QMIV_IVMSSSIM);
   if(need_search) { QMIV_TRY(cps_rows_.ensure(ctx_, (size_t)2 * S.H * 3 * sizeof(uint32_t))); }
   if(need_scp) { QMIV_TRY(scp_.ensure(ctx_, (size_t)2 * 3 * S.W * S.H * S.esz)); }
-  if(need_ssim && !gen_)
-  {
-    // moment slots: 0, 1 = IV-SSIM directions (written by the search), 2 = SSIM / MS-SSIM pair,
-    // 3, 4 = IV-MS-SSIM pairs
-    const int slots = (mask & QMIV_IVMSSSIM) ? 5 : (mask & (QMIV_SSIM | QMIV_MSSSIM)) ? 3 : 2;
-    QMIV_TRY(mom_.ensure(ctx_, (size_t)slots * mom_slot_elems() * sizeof(uint32_t)));
-  }
+  // moments of the two IV-SSIM directions, written by the search
+  if((mask & QMIV_IVSSIM) && !gen_) { QMIV_TRY(mom_.ensure(ctx_, (size_t)2 * mom_slot_elems() * sizeof(uint32_t))); }
   if(prm_.erp)
   {
     QMIV_TRY(ws_.ensure(ctx_, (size_t)S.H * sizeof(double)));
@@ -205,8 +200,8 @@ qmiv_status PairPipeline::prepare(uint32_t mask, bool want_scp, bool host_frames
   {
     if(nx_[0] < 1 || ny_[0] < 1) { return fail(QMIV_ERR_INVALID_ARG, "picture smaller than one 8x8 SSIM window"); }
     QMIV_TRY(rowsum_.ensure(ctx_, (size_t)kMaxSsimSlots * 3 * ny_[0] * sizeof(double)));
-    // window values of up to 9 pool jobs (one flush) at scale 0, reused by later flushes
-    QMIV_TRY(win_.ensure(ctx_, (size_t)9 * pool_win_elems(nx_[0], ny_[0]) * sizeof(double)));
+    if(need_ms && ns_ < 1) { return fail(QMIV_ERR_INVALID_ARG, "picture too small for MS-SSIM (needs >= 32x32)"); }
+    QMIV_TRY(win_.ensure(ctx_, ssim_win_elems(mask, ns_, nx_, ny_) * sizeof(double)));
   }
   if(need_ssim && gen_)
   {
@@ -374,102 +369,25 @@ qmiv_status PairPipeline::enqueue_t(const Img& in0, const Img& in1, uint32_t mas
   }
   else
   {
-    double* rowsum = rowsum_.as<double>();
-    // window pooling of up to three pictures pairs (x 3 components) from their moments, one launch
-    SsimPoolArgs pool{};
-    auto add_pool = [&](const Moments& m, int scale, int slot, int calc_l, int use_ws) {
-      for(int c = 0; c < 3; c++)
-      {
-        SsimPoolJob& J = pool.job[pool.njobs];
-        J.win = win_.as<double>() + (size_t)pool.njobs * pool_win_elems(nx_[0], ny_[0]);
-        pool.njobs++;
-        J.mom = m.p + (size_t)c * 5 * m.plane(); J.plane = m.plane(); J.pitch = m.pitch;
-        J.C1 = C1_; J.C2 = C2_;
-        J.nx = nx_[scale]; J.ny = ny_[scale]; J.calc_l = calc_l; J.wide = shape_.bitdepth > 12 ? 1 : 0;
-        J.row_sum = rowsum + (size_t)slot * 3 * ny_[0] + (size_t)c * ny_[scale];  // finalize reads [c][ny_scale]
-      }
-      fa.slot[slot].row_sum = rowsum + (size_t)slot * 3 * ny_[0];
-      fa.slot[slot].nx = nx_[scale]; fa.slot[slot].ny = ny_[scale]; fa.slot[slot].use_ws = use_ws;
-      fa.slot[slot].ws_base = 4; fa.slot[slot].ws_step = 4;  // window row j covers rows 4j..4j+7 (xIVSSIM.cpp:153)
-    };
-    auto flush_pool = [&]() -> qmiv_status {
-      if(pool.njobs == 0) { return QMIV_OK; }
-      const int t = prof_begin(s);
-      QMIV_CUDA(launch_ssim_pool(pool, s));
-      prof_end(s, QMIV_STAGE_SSIM_ROWS, t);
-      pool.njobs = 0;
-      return QMIV_OK;
-    };
-    auto moments = [&](const Img& a, const Img& b, int W, int H, const Moments& m, const MutImg* down_a,
-                       const MutImg* down_b) -> qmiv_status {
-      SsimMomArgs ma{};
-      ma.a = a; ma.b = b; ma.W = W; ma.H = H; ma.clip = clip; ma.mom = m;
-      if(down_a) { ma.down_a = *down_a; }
-      if(down_b) { ma.down_b = *down_b; }
-      const int t = prof_begin(s);
-      QMIV_CUDA(launch_ssim_moments<T>(ma, s));
+    const uint32_t family = mask & kSsimFamily;
+    if(family)
+    {
+      SsimPairArgs sa{};
+      sa.in0 = in0; sa.in1 = in1;
+      if(need_scp) { sa.scp0 = img444(scp(0), S.W, S.H, S.esz); sa.scp1 = img444(scp(1), S.W, S.H, S.esz); }
+      sa.mask = family; sa.W = S.W; sa.H = S.H; sa.esz = (int32_t)S.esz; sa.bitdepth = S.bitdepth; sa.clip = clip;
+      sa.ns = ns_; sa.C1 = C1_; sa.C2 = C2_; sa.use_ws = prm_.erp ? 1 : 0;
+      for(int k = 0; k < 5; k++) { sa.nx[k] = nx_[k]; sa.ny[k] = ny_[k]; }
+      sa.mom[0] = mom_at(0, 0); sa.mom[1] = mom_at(1, 0);
+      sa.rowsum = rowsum_.as<double>(); sa.win = win_.as<double>(); sa.pyr = pyr_.as<char>();
+      SsimJobs jobs;
+      add_ssim_jobs(sa, jobs, fa);
+      int t = prof_begin(s);
+      QMIV_CUDA(launch_ssim_jobs(jobs, s, false));
       prof_end(s, QMIV_STAGE_SSIM_WIN, t);
-      return QMIV_OK;
-    };
-
-    const Img scp0 = need_scp ? img444(scp(0), S.W, S.H, S.esz) : Img{};
-    const Img scp1 = need_scp ? img444(scp(1), S.W, S.H, S.esz) : Img{};
-    const int use_ws = prm_.erp ? 1 : 0;
-    if(mask & QMIV_IVSSIM)  // moments written by the search: (In0, SCP1) = T2R, (In1, SCP0) = R2T (xIVSSIM.cpp:46-47)
-    {
-      add_pool(mom_at(0, 0), 0, kSlotIvT2R, 1, use_ws);
-      add_pool(mom_at(1, 0), 0, kSlotIvR2T, 1, use_ws);
-    }
-    if(mask & QMIV_SSIM)  // xSSIM.h:83
-    {
-      QMIV_TRY(moments(in0, in1, S.W, S.H, mom_at(2, 0), nullptr, nullptr));
-      if(pool.njobs + 3 > 9) { QMIV_TRY(flush_pool()); }
-      add_pool(mom_at(2, 0), 0, kSlotSsim, 1, 0);
-    }
-    QMIV_TRY(flush_pool());
-    if(mask & (QMIV_MSSSIM | QMIV_IVMSSSIM))                                                                      // xSSIM.cpp:230-256
-    {
-      // pyramid levels 1..ns-1 of In0, In1, SCP0, SCP1
-      size_t lv = 0;
-      for(int s2 = 1; s2 < ns_; s2++) { lv += (size_t)(S.W >> s2) * (S.H >> s2) * 3; }
-      auto level_base = [&](int img, int scale) -> char* {
-        size_t o = (size_t)img * lv;
-        for(int s2 = 1; s2 < scale; s2++) { o += (size_t)(S.W >> s2) * (S.H >> s2) * 3; }
-        return pyr_.as<char>() + o * S.esz;
-      };
-      auto level_img = [&](int img, int scale) -> Img {
-        if(scale == 0) { return img == 0 ? in0 : img == 1 ? in1 : img == 2 ? scp0 : scp1; }
-        return img444(level_base(img, scale), S.W >> scale, S.H >> scale, S.esz);
-      };
-      for(int sc = 0; sc < ns_; sc++)
-      {
-        const int Ws = S.W >> sc, Hs = S.H >> sc;
-        const bool last = sc == ns_ - 1;
-        bool written[4] = { false, false, false, false };
-        auto down = [&](int img, MutImg& m) -> const MutImg* {
-          if(last || written[img]) { return nullptr; }
-          written[img] = true;
-          m = mut444(level_base(img, sc + 1), S.W >> (sc + 1), S.H >> (sc + 1), S.esz);
-          return &m;
-        };
-        MutImg m0, m1, m2, m3, m4, m5;
-        if(mask & QMIV_MSSSIM)
-        {
-          const MutImg* d0 = down(0, m0); const MutImg* d1 = down(1, m1);
-          QMIV_TRY(moments(level_img(0, sc), level_img(1, sc), Ws, Hs, mom_at(2, sc), d0, d1));
-          add_pool(mom_at(2, sc), sc, kSlotMs + sc, last ? 1 : 0, 0);
-        }
-        if(mask & QMIV_IVMSSSIM)  // xIVSSIM.cpp:77-78, no ERP weighting
-        {
-          const MutImg* d0 = down(0, m2); const MutImg* d3 = down(3, m3);
-          QMIV_TRY(moments(level_img(0, sc), level_img(3, sc), Ws, Hs, mom_at(3, sc), d0, d3));
-          add_pool(mom_at(3, sc), sc, kSlotIvmsT2R + sc, last ? 1 : 0, 0);
-          const MutImg* d1 = down(1, m4); const MutImg* d2 = down(2, m5);
-          QMIV_TRY(moments(level_img(1, sc), level_img(2, sc), Ws, Hs, mom_at(4, sc), d1, d2));
-          add_pool(mom_at(4, sc), sc, kSlotIvmsR2T + sc, last ? 1 : 0, 0);
-        }
-        QMIV_TRY(flush_pool());
-      }
+      t = prof_begin(s);
+      QMIV_CUDA(launch_ssim_jobs(jobs, s, true));
+      prof_end(s, QMIV_STAGE_SSIM_ROWS, t);
     }
   }
 
@@ -498,7 +416,8 @@ qmiv_status PairPipeline::enqueue_ssim_gen(const Img& in0, const Img& in1, const
   double* rowsum = rowsum_.as<double>();
   const size_t wstride = pool_win_elems(gnx_[0], gny_[0]);
   SsimGenArgs ga{};
-  SsimPoolArgs rows{};
+  JobArgs<SsimRowJob, kMaxRowJobs> rows{};
+  int nrows = 0;
   auto add = [&](const Img& a, const Img& b, int scale, int slot, int calc_l, int use_ws) {
     for(int c = 0; c < 3; c++)
     {
@@ -508,11 +427,10 @@ qmiv_status PairPipeline::enqueue_ssim_gen(const Img& in0, const Img& in1, const
       J.x0 = gfirst_; J.y0 = gfirst_; J.nx = gnx_[scale]; J.ny = gny_[scale];
       J.calc_l = calc_l; J.clip = clip; J.esz = (int32_t)S.esz; J.small_range = S.maxv < 0x4000; J.flags = &out_.as<PairOut>()->flags; J.C1 = C1_; J.C2 = C2_;
       J.win = win_.as<double>() + (size_t)ga.njobs * wstride;
-      SsimPoolJob& P = rows.job[rows.njobs];
-      P = SsimPoolJob{};
+      SsimRowJob& P = rows.job[nrows];
       P.win = J.win; P.nx = J.nx; P.ny = J.ny;
       P.row_sum = rowsum + (size_t)slot * 3 * gny_[0] + (size_t)c * gny_[scale];   // finalize reads [c][ny_scale]
-      ga.njobs++; rows.njobs++;
+      ga.njobs++; nrows++;
     }
     SsimSlot& sl = fa.slot[slot];
     sl.row_sum = rowsum + (size_t)slot * 3 * gny_[0];
@@ -525,9 +443,9 @@ qmiv_status PairPipeline::enqueue_ssim_gen(const Img& in0, const Img& in1, const
     QMIV_CUDA(launch_ssim_gen(ga, prm_.ssim_mode, N, prm_.ssim_stride, prm_.ssim_border, s));
     prof_end(s, QMIV_STAGE_SSIM_WIN, t);
     t = prof_begin(s);
-    QMIV_CUDA(launch_ssim_rows(rows, s));
+    QMIV_CUDA(launch_ssim_rows(rows, nrows, s));
     prof_end(s, QMIV_STAGE_SSIM_ROWS, t);
-    ga.njobs = 0; rows.njobs = 0;
+    ga.njobs = 0; nrows = 0;
     return QMIV_OK;
   };
 

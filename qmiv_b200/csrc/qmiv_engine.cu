@@ -6,7 +6,7 @@
 //   reduce        one CTA per pair                                        (k_reduce_multi)
 //   CPS           one persistent launch per (R, sample size, tile height) over a work list of the
 //                 tiles of all its pairs                                   (k_cps_multi)
-//   SSIM          per scale: moments of all pairs, then every window row of every (pair, component)
+//   SSIM          windows of all pairs at scale 0, the smaller scales, their windows, every window row
 //   finalize      one CTA per (pair, pooling chain)                       (k_finalize_multi)
 //   results       one device-to-host copy of all pairs' PairOut
 //
@@ -44,13 +44,6 @@ Img img444(const void* base, int32_t W, int32_t H, size_t esz)
   }
   return im;
 }
-MutImg mut444(void* base, int32_t W, int32_t H, size_t esz)
-{
-  MutImg im{};
-  for(int c = 0; c < 3; c++) { im.p[c] = static_cast<char*>(base) + (size_t)c * W * H * esz; im.pitch[c] = W; }
-  return im;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------------------------
@@ -306,14 +299,11 @@ qmiv_status Engine::submit(const qmiv_pair_desc* pairs, int32_t n)
     if(p.need_scp) { p.scp = take((size_t)2 * 3 * S.W * S.H * S.esz); }
     if(p.need_ssim)
     {
-      const int slots = (p.mask & QMIV_IVMSSSIM) ? 5 : (p.mask & (QMIV_SSIM | QMIV_MSSSIM)) ? 3 : 2;
+      // moments of the two IV-SSIM directions, written by the search
       p.mom_slot = mom_slot_elems(S);
-      p.mom = take((size_t)slots * p.mom_slot * sizeof(uint32_t));
+      if(p.mask & QMIV_IVSSIM) { p.mom = take((size_t)2 * p.mom_slot * sizeof(uint32_t)); }
       p.rowsum = take((size_t)kMaxSsimSlots * 3 * K.ny[0] * sizeof(double));
-      // window values of the pair's scale-0 pool jobs, reused by the MS-SSIM scales
-      const int jobs0 = 3 * (((p.mask & QMIV_IVSSIM) ? 2 : 0) + ((p.mask & QMIV_SSIM) ? 1 : 0) +
-                             ((p.mask & QMIV_MSSSIM) ? 1 : 0) + ((p.mask & QMIV_IVMSSSIM) ? 2 : 0));
-      p.win = take((size_t)jobs0 * pool_win_elems(K.nx[0], K.ny[0]) * sizeof(double));
+      p.win = take(ssim_win_elems(p.mask, K.ns, K.nx, K.ny) * sizeof(double));
     }
     if(p.need_ms)
     {
@@ -570,11 +560,11 @@ size_t Engine::mom_slot_elems(const Shape& S)
   return 3 * 5 * nby * ((nbx + 7) & ~(size_t)7);
 }
 
-Moments Engine::mom_at(const Shape& S, const PairSlot& p, char* dbase, int slot, int scale)
+Moments Engine::mom_at(const Shape& S, const PairSlot& p, char* dbase, int slot)
 {
   Moments m{};
-  m.nbx = ((S.W >> scale) + 3) / 4;
-  m.nby = ((S.H >> scale) + 3) / 4;
+  m.nbx = (S.W + 3) / 4;
+  m.nby = (S.H + 3) / 4;
   m.pitch = (m.nbx + 7) & ~7;
   m.p = reinterpret_cast<uint32_t*>(dbase + p.mom) + (size_t)slot * p.mom_slot;
   return m;
@@ -604,10 +594,6 @@ qmiv_status Engine::build_tables(int first, int n, const std::vector<PairKind*>&
     const PairKind& K = *kind[i];
     T.cps_groups[CpsGroupKey{ K.R, (int)K.S.esz, K.wy }].push_back(i);
   }
-  int max_ns = 0;
-  for(int i = first; i < first + n; i++) { if(slots_[i].need_ms) { max_ns = std::max(max_ns, kind[i]->ns); } }
-  T.phases = std::max(1, max_ns);
-
   size_t off = 0;
   auto place = [&](size_t bytes, size_t align) { off = align_sz(off, align); const size_t o = off; off += bytes; return o; };
   T.prepass_off[0] = place(sizeof(PrepassArgs) * T.prepass_idx[0].size(), 64);
@@ -618,18 +604,23 @@ qmiv_status Engine::build_tables(int first, int n, const std::vector<PairKind*>&
   T.cps_off = place(cps_desc_bytes() * ncps, 64);
   T.prefix_off = place(sizeof(int32_t) * (ncps + T.cps_groups.size()), 16);
   T.fin_off = place(sizeof(FinalizeArgs) * (size_t)n, 64);
-  size_t mom_jobs = 0, pool_jobs = 0, fin_jobs = 0;
+  size_t npool = 0, nimg0 = 0, nimgn = 0, npyr = 0, fin_jobs = 0;
   for(int i = first; i < first + n; i++)
   {
     const PairSlot& p = slots_[i];
+    const size_t per_scale = ((p.mask & QMIV_MSSSIM) ? 1 : 0) + ((p.mask & QMIV_IVMSSSIM) ? 2 : 0);
     const size_t ns = p.need_ms ? (size_t)kind[i]->ns : 0;
-    mom_jobs += ((p.mask & QMIV_SSIM) ? 1 : 0) + ns * (((p.mask & QMIV_MSSSIM) ? 1 : 0) + ((p.mask & QMIV_IVMSSSIM) ? 2 : 0));
-    pool_jobs += 3 * (((p.mask & QMIV_IVSSIM) ? 2 : 0) + ((p.mask & QMIV_SSIM) ? 1 : 0) +
-                      ns * (((p.mask & QMIV_MSSSIM) ? 1 : 0) + ((p.mask & QMIV_IVMSSSIM) ? 2 : 0)));
+    npool += (p.mask & QMIV_IVSSIM) ? 6 : 0;
+    nimg0 += 3 * (((p.mask & QMIV_SSIM) ? 1 : 0) + (ns > 0 ? per_scale : 0));
+    nimgn += ns > 1 ? 3 * (ns - 1) * per_scale : 0;
+    npyr += ns > 2 ? (size_t)((p.mask & QMIV_IVMSSSIM) ? 12 : 6) : 0;
     fin_jobs += 3 + 6 + 3 * kMaxSsimSlots + 1;
   }
-  T.mom_off = place(sizeof(SsimMomArgs) * mom_jobs, 64);
-  T.pool_off = place(sizeof(SsimPoolJob) * pool_jobs, 64);
+  T.pool_off = place(sizeof(SsimPoolJob) * npool, 64);
+  T.img0_off = place(sizeof(SsimImgJob) * nimg0, 64);
+  T.imgn_off = place(sizeof(SsimImgJob) * nimgn, 64);
+  T.pyr_off = place(sizeof(SsimPyrJob) * npyr, 64);
+  T.rows_off = place(sizeof(SsimRowJob) * (npool + nimg0 + nimgn), 64);
   T.finjob_off = place(sizeof(FinJob) * fin_jobs, 16);
   T.bytes = align_sz(off, 256);
   return QMIV_OK;
@@ -701,7 +692,7 @@ void Engine::fill_tables(int n, const std::vector<PairKind*>& kind, const std::v
           ca.scp0 = dbase + p.scp;
           ca.scp1 = dbase + p.scp + (size_t)3 * K.S.W * K.S.H * K.S.esz;
         }
-        if(p.mask & QMIV_IVSSIM) { ca.mom[0] = mom_at(K.S, p, dbase, 0, 0); ca.mom[1] = mom_at(K.S, p, dbase, 1, 0); }
+        if(p.mask & QMIV_IVSSIM) { ca.mom[0] = mom_at(K.S, p, dbase, 0); ca.mom[1] = mom_at(K.S, p, dbase, 1); }
         CpsPairPlan plan{};
         cps_describe(cdesc + di * cps_desc_bytes(), ca, K.R, (int)K.S.esz, K.wy, &plan);
         prefix[pi++] = tiles;
@@ -715,29 +706,43 @@ void Engine::fill_tables(int n, const std::vector<PairKind*>& kind, const std::v
       T.cps_launch.push_back(L);
     }
   }
-  // SSIM moments / pool jobs per phase, finalize
-  SsimMomArgs* mj = reinterpret_cast<SsimMomArgs*>(h + T.mom_off);
-  SsimPoolJob* pj = reinterpret_cast<SsimPoolJob*>(h + T.pool_off);
+  // SSIM windows and row sums, finalize
   FinalizeArgs* fa = reinterpret_cast<FinalizeArgs*>(h + T.fin_off);
-  size_t nm = 0, np = 0;
-  T.phase.assign(T.phases, Phase{});
-  for(int ph = 0; ph < T.phases; ph++)
+  SsimTables& st = T.ssim;
+  st = SsimTables{};
+  for(int i = first; i < first + n; i++)
   {
-    Phase& PH = T.phase[ph];
-    for(int esz = 0; esz < 2; esz++)
+    const PairKind& K = *kind[i];
+    const PairSlot& p = slots_[i];
+    const Shape& S = K.S;
+    if(!p.need_ssim) { continue; }
+    SsimPairArgs sa{};
+    sa.in0 = in0[i]; sa.in1 = in1[i];
+    if(p.need_scp)
     {
-      PH.mom_first[esz] = nm;
-      for(int i = first; i < first + n; i++)
-      {
-        if((kind[i]->S.esz == 1 ? 0 : 1) != esz) { continue; }
-        add_moment_jobs(i, *kind[i], ph, in0[i], in1[i], dbase, mj, nm, PH);
-      }
-      PH.mom_count[esz] = nm - PH.mom_first[esz];
+      sa.scp0 = img444(dbase + p.scp, S.W, S.H, S.esz);
+      sa.scp1 = img444(dbase + p.scp + (size_t)3 * S.W * S.H * S.esz, S.W, S.H, S.esz);
     }
-    PH.pool_first = np;
-    for(int i = first; i < first + n; i++) { add_pool_jobs(i, *kind[i], ph, dbase, pj, np, PH, fa[i - first]); }
-    PH.pool_count = np - PH.pool_first;
+    sa.mask = p.mask & kSsimFamily; sa.W = S.W; sa.H = S.H; sa.esz = (int32_t)S.esz; sa.bitdepth = S.bitdepth; sa.clip = clip_of(K);
+    sa.ns = K.ns; sa.C1 = K.C1; sa.C2 = K.C2; sa.use_ws = prm_.erp ? 1 : 0;
+    for(int k = 0; k < 5; k++) { sa.nx[k] = K.nx[k]; sa.ny[k] = K.ny[k]; }
+    if(p.mask & QMIV_IVSSIM) { sa.mom[0] = mom_at(S, p, dbase, 0); sa.mom[1] = mom_at(S, p, dbase, 1); }
+    sa.rowsum = reinterpret_cast<double*>(dbase + p.rowsum); sa.win = reinterpret_cast<double*>(dbase + p.win); sa.pyr = dbase + p.pyr;
+    SsimJobs q;
+    add_ssim_jobs(sa, q, fa[i - first]);
+    std::memcpy(h + T.pool_off + sizeof(SsimPoolJob) * st.npool, q.pool.job, sizeof(SsimPoolJob) * q.npool);
+    std::memcpy(h + T.img0_off + sizeof(SsimImgJob) * st.nimg0, q.img0.job, sizeof(SsimImgJob) * q.nimg0);
+    std::memcpy(h + T.imgn_off + sizeof(SsimImgJob) * st.nimgn, q.imgn.job, sizeof(SsimImgJob) * q.nimgn);
+    std::memcpy(h + T.pyr_off + sizeof(SsimPyrJob) * st.npyr, q.pyr.job, sizeof(SsimPyrJob) * q.npyr);
+    std::memcpy(h + T.rows_off + sizeof(SsimRowJob) * st.nrows, q.rows.job, sizeof(SsimRowJob) * q.nrows);
+    st.npool += q.npool; st.nimg0 += q.nimg0; st.nimgn += q.nimgn; st.npyr += q.npyr; st.nrows += q.nrows;
+    st.dims.add(q);
   }
+  st.pool = reinterpret_cast<const SsimPoolJob*>(d + T.pool_off);
+  st.img0 = reinterpret_cast<const SsimImgJob*>(d + T.img0_off);
+  st.imgn = reinterpret_cast<const SsimImgJob*>(d + T.imgn_off);
+  st.pyr = reinterpret_cast<const SsimPyrJob*>(d + T.pyr_off);
+  st.rows = reinterpret_cast<const SsimRowJob*>(d + T.rows_off);
   FinJob* fj = reinterpret_cast<FinJob*>(h + T.finjob_off);
   size_t nf = 0;
   T.fin_smem = 0;
@@ -764,113 +769,6 @@ void Engine::fill_tables(int n, const std::vector<PairKind*>& kind, const std::v
   T.d_prepass[0] = reinterpret_cast<const PrepassArgs*>(d + T.prepass_off[0]);
   T.d_prepass[1] = reinterpret_cast<const PrepassArgs*>(d + T.prepass_off[1]);
   T.d_reduce = reinterpret_cast<const ReduceArgs*>(d + T.reduce_off);
-  T.d_mom = reinterpret_cast<const SsimMomArgs*>(d + T.mom_off);
-  T.d_pool = reinterpret_cast<const SsimPoolJob*>(d + T.pool_off);
-}
-
-// SSIM moments of phase (scale) ph of pair i: plain SSIM at scale 0, MS-SSIM / IV-MS-SSIM scales
-// with the next pyramid level written on the way (xSSIM.cpp:230-256)
-void Engine::add_moment_jobs(int i, const PairKind& K, int ph, const Img& a0, const Img& a1, char* dbase,
-                             SsimMomArgs* mj, size_t& nm, Phase& PH)
-{
-  const PairSlot& p = slots_[i];
-  const Shape& S = K.S;
-  const int ns = p.need_ms ? K.ns : 0;
-  const Img scp0 = p.need_scp ? img444(dbase + p.scp, S.W, S.H, S.esz) : Img{};
-  const Img scp1 = p.need_scp ? img444(dbase + p.scp + (size_t)3 * S.W * S.H * S.esz, S.W, S.H, S.esz) : Img{};
-  auto level_base = [&](int img, int scale) -> char* {
-    size_t o = (size_t)img * p.pyr_lv;
-    for(int s2 = 1; s2 < scale; s2++) { o += (size_t)(S.W >> s2) * (S.H >> s2) * 3; }
-    return dbase + p.pyr + o * S.esz;
-  };
-  auto level_img = [&](int img, int scale) -> Img {
-    if(scale == 0) { return img == 0 ? a0 : img == 1 ? a1 : img == 2 ? scp0 : scp1; }
-    return img444(level_base(img, scale), S.W >> scale, S.H >> scale, S.esz);
-  };
-  const uint32_t clip = clip_of(K);
-  auto push = [&](const Img& x, const Img& y, int W, int H, const Moments& m, const MutImg* dx, const MutImg* dy) {
-    SsimMomArgs& a = mj[nm++];
-    a.a = x; a.b = y; a.W = W; a.H = H; a.clip = clip; a.mom = m;
-    if(dx) { a.down_a = *dx; }
-    if(dy) { a.down_b = *dy; }
-    PH.mom_max_nbx = std::max(PH.mom_max_nbx, m.nbx);
-    PH.mom_max_nby = std::max(PH.mom_max_nby, m.nby);
-  };
-  if(ph == 0 && (p.mask & QMIV_SSIM)) { push(a0, a1, S.W, S.H, mom_at(S, p, dbase, 2, 0), nullptr, nullptr); }
-  if(ph < ns)
-  {
-    const int sc = ph;
-    const int Ws = S.W >> sc, Hs = S.H >> sc;
-    const bool last = sc == ns - 1;
-    bool written[4] = { false, false, false, false };
-    MutImg m[6];
-    int mi = 0;
-    auto down = [&](int img) -> const MutImg* {
-      if(last || written[img]) { return nullptr; }
-      written[img] = true;
-      m[mi] = mut444(level_base(img, sc + 1), S.W >> (sc + 1), S.H >> (sc + 1), S.esz);
-      return &m[mi++];
-    };
-    if(p.mask & QMIV_MSSSIM)
-    {
-      const MutImg* d0 = down(0); const MutImg* d1 = down(1);
-      push(level_img(0, sc), level_img(1, sc), Ws, Hs, mom_at(S, p, dbase, 2, sc), d0, d1);
-    }
-    if(p.mask & QMIV_IVMSSSIM)  // xIVSSIM.cpp:77-78, no ERP weighting
-    {
-      const MutImg* d0 = down(0); const MutImg* d3 = down(3);
-      push(level_img(0, sc), level_img(3, sc), Ws, Hs, mom_at(S, p, dbase, 3, sc), d0, d3);
-      const MutImg* d1 = down(1); const MutImg* d2 = down(2);
-      push(level_img(1, sc), level_img(2, sc), Ws, Hs, mom_at(S, p, dbase, 4, sc), d1, d2);
-    }
-  }
-}
-
-void Engine::add_pool_jobs(int i, const PairKind& K, int ph, char* dbase, SsimPoolJob* pj, size_t& np, Phase& PH,
-                           FinalizeArgs& fa)
-{
-  const PairSlot& p = slots_[i];
-  if(!p.need_ssim) { return; }
-  const Shape& S = K.S;
-  const int ns = p.need_ms ? K.ns : 0;
-  double* rowsum = reinterpret_cast<double*>(dbase + p.rowsum);
-  double* win = reinterpret_cast<double*>(dbase + p.win);
-  int jobs_here = 0;
-  auto add = [&](const Moments& m, int scale, int slot, int calc_l, int use_ws) {
-    for(int c = 0; c < 3; c++)
-    {
-      SsimPoolJob& J = pj[np++];
-      J.win = win + (size_t)(jobs_here++) * pool_win_elems(K.nx[0], K.ny[0]);
-      J.C1 = K.C1; J.C2 = K.C2;
-      J.mom = m.p + (size_t)c * 5 * m.plane(); J.plane = m.plane(); J.pitch = m.pitch;
-      J.nx = K.nx[scale]; J.ny = K.ny[scale]; J.calc_l = calc_l; J.wide = S.bitdepth > 12 ? 1 : 0;
-      J.row_sum = rowsum + (size_t)slot * 3 * K.ny[0] + (size_t)c * K.ny[scale];  // finalize reads [c][ny_scale]
-      assert(pool_job_aligned(J));
-      PH.pool_max_nx = std::max(PH.pool_max_nx, J.nx);
-      PH.pool_max_ny = std::max(PH.pool_max_ny, J.ny);
-    }
-    fa.slot[slot].row_sum = rowsum + (size_t)slot * 3 * K.ny[0];
-    fa.slot[slot].nx = K.nx[scale]; fa.slot[slot].ny = K.ny[scale]; fa.slot[slot].use_ws = use_ws;
-    fa.slot[slot].ws_base = 4; fa.slot[slot].ws_step = 4;  // window row j covers rows 4j..4j+7 (xIVSSIM.cpp:153)
-  };
-  const int use_ws = prm_.erp ? 1 : 0;
-  if(ph == 0 && (p.mask & QMIV_IVSSIM))  // (In0, SCP1) = T2R, (In1, SCP0) = R2T (xIVSSIM.cpp:46-47)
-  {
-    add(mom_at(S, p, dbase, 0, 0), 0, kSlotIvT2R, 1, use_ws);
-    add(mom_at(S, p, dbase, 1, 0), 0, kSlotIvR2T, 1, use_ws);
-  }
-  if(ph == 0 && (p.mask & QMIV_SSIM)) { add(mom_at(S, p, dbase, 2, 0), 0, kSlotSsim, 1, 0); }
-  if(ph < ns)
-  {
-    const int sc = ph;
-    const bool last = sc == ns - 1;
-    if(p.mask & QMIV_MSSSIM) { add(mom_at(S, p, dbase, 2, sc), sc, kSlotMs + sc, last ? 1 : 0, 0); }
-    if(p.mask & QMIV_IVMSSSIM)
-    {
-      add(mom_at(S, p, dbase, 3, sc), sc, kSlotIvmsT2R + sc, last ? 1 : 0, 0);
-      add(mom_at(S, p, dbase, 4, sc), sc, kSlotIvmsR2T + sc, last ? 1 : 0, 0);
-    }
-  }
 }
 
 qmiv_status Engine::launch_all(const Tables& T, cudaStream_t s)
@@ -892,22 +790,14 @@ qmiv_status Engine::launch_all(const Tables& T, cudaStream_t s)
     QMIV_CUDA(launch_cps_multi(L.d_desc, L.d_prefix, L.npairs, L.ntiles, L.R, L.wy, L.esz, L.raw_cap, L.smem, s));
     prof_end(s, QMIV_STAGE_CPS, t);
   }
-  for(int ph = 0; ph < T.phases; ph++)
+  if(T.ssim.nrows > 0)
   {
-    const Phase& PH = T.phase[ph];
-    if(PH.mom_count[0] + PH.mom_count[1] > 0)
-    {
-      const int t = prof_begin(s);
-      QMIV_CUDA(launch_ssim_moments_multi<uint8_t>(T.d_mom + PH.mom_first[0], (int)PH.mom_count[0], PH.mom_max_nbx, PH.mom_max_nby, s));
-      QMIV_CUDA(launch_ssim_moments_multi<uint16_t>(T.d_mom + PH.mom_first[1], (int)PH.mom_count[1], PH.mom_max_nbx, PH.mom_max_nby, s));
-      prof_end(s, QMIV_STAGE_SSIM_WIN, t);
-    }
-    if(PH.pool_count > 0)
-    {
-      const int t = prof_begin(s);
-      QMIV_CUDA(launch_ssim_pool_multi(T.d_pool + PH.pool_first, (int)PH.pool_count, PH.pool_max_nx, PH.pool_max_ny, s));
-      prof_end(s, QMIV_STAGE_SSIM_ROWS, t);
-    }
+    int t = prof_begin(s);
+    QMIV_CUDA(launch_ssim_tables(T.ssim, s, false));
+    prof_end(s, QMIV_STAGE_SSIM_WIN, t);
+    t = prof_begin(s);
+    QMIV_CUDA(launch_ssim_tables(T.ssim, s, true));
+    prof_end(s, QMIV_STAGE_SSIM_ROWS, t);
   }
   {
     const int t = prof_begin(s);

@@ -59,15 +59,6 @@ struct CpsLaunch
   size_t         smem = 0;
 };
 
-// SSIM work of one scale: moment jobs per sample size, then pool jobs
-struct Phase
-{
-  size_t mom_first[2] = { 0, 0 }, mom_count[2] = { 0, 0 };
-  int    mom_max_nbx = 0, mom_max_nby = 0;
-  size_t pool_first = 0, pool_count = 0;
-  int    pool_max_nx = 0, pool_max_ny = 0;
-};
-
 // Argument tables of one set of pairs: host layout, device pointers, launch shapes.
 struct Tables
 {
@@ -77,17 +68,14 @@ struct Tables
   std::vector<int> prepass_idx[2];
   int    prepass_max_rows[2] = { 0, 0 };
   size_t prepass_off[2] = { 0, 0 }, reduce_off = 0, cps_off = 0, prefix_off = 0, fin_off = 0;
-  size_t mom_off = 0, pool_off = 0, finjob_off = 0;
+  size_t pool_off = 0, img0_off = 0, imgn_off = 0, pyr_off = 0, rows_off = 0, finjob_off = 0;
   std::map<CpsGroupKey, std::vector<int>> cps_groups;
   std::vector<CpsLaunch> cps_launch;
-  int    phases = 1;
-  std::vector<Phase> phase;
+  SsimTables ssim;
   int    fin_jobs = 0;
   size_t fin_smem = 0;
   const PrepassArgs*  d_prepass[2] = { nullptr, nullptr };
   const ReduceArgs*   d_reduce = nullptr;
-  const SsimMomArgs*  d_mom = nullptr;
-  const SsimPoolJob*  d_pool = nullptr;
   const FinalizeArgs* d_fin = nullptr;
   const FinJob*       d_finjobs = nullptr;
 };
@@ -117,14 +105,10 @@ private:
   qmiv_status build_tables(int first, int n, const std::vector<PairKind*>& kind, Tables& T);
   void        fill_tables(int n, const std::vector<PairKind*>& kind, const std::vector<Img>& in0,
                           const std::vector<Img>& in1, char* dbase, Tables& T, char* h, char* d);
-  void        add_moment_jobs(int i, const PairKind& K, int ph, const Img& a0, const Img& a1, char* dbase, SsimMomArgs* mj,
-                              size_t& nm, Phase& PH);
-  void        add_pool_jobs(int i, const PairKind& K, int ph, char* dbase, SsimPoolJob* pj, size_t& np, Phase& PH,
-                            FinalizeArgs& fa);
   qmiv_status launch_all(const Tables& T, cudaStream_t s);
   uint32_t    clip_of(const PairKind& K) const;
   static size_t  mom_slot_elems(const Shape& S);
-  static Moments mom_at(const Shape& S, const PairSlot& p, char* dbase, int slot, int scale);
+  static Moments mom_at(const Shape& S, const PairSlot& p, char* dbase, int slot);
   int  prof_begin(cudaStream_t s);
   void prof_end(cudaStream_t s, int stage, int token);
   void harvest_profile();

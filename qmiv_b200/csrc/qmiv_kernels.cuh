@@ -70,14 +70,32 @@ struct CpsArgs
 // ---------------------------------------------------------------------------------------------
 // block SSIM
 // ---------------------------------------------------------------------------------------------
-// moments of an image pair (+ fused 2x2 downsampling of both inputs for the next MS-SSIM scale)
-struct SsimMomArgs
+// windows of one component of a picture pair, straight from the pictures, and the 2x2 means of both
+// for the next MS-SSIM scale
+enum { kLoadAny = 0, kLoadRow = 1, kLoadSub = 2 };   // any plane / full-size plane / 4:2:0 chroma
+struct SsimImgJob
 {
-  Img      a, b;               // a = "Tst" picture, b = "Ref" picture of xSSIM::xCalcPicSSIM
-  int32_t  W, H;
-  uint32_t clip;
-  Moments  mom;
-  MutImg   down_a, down_b;     // outputs ((W>>1) x (H>>1), 4:4:4) or null planes
+  double      C1, C2;          // (0.01 Max)^2, (0.03 Max)^2 of the pair's bit depth
+  const void* a;               // plane of the "Tst" picture of xSSIM::xCalcPicSSIM
+  const void* b;               // ... of the "Ref" picture
+  double*     win;             // window values [ceil(ny / 32)][nx][32] (pool_win_elems)
+  void*       down_a;          // (W >> 1) x (H >> 1), pitch W >> 1, or null
+  void*       down_b;
+  int32_t     pitch_a, pitch_b;
+  int32_t     W, H;            // 4:4:4 size
+  int32_t     nx, ny;          // windows per row / column
+  uint32_t    clip;
+  int8_t      sxa, sya, sxb, syb, load_a, load_b, vec_a, vec_b;
+  int8_t      esz, calc_l, wide, down_vec;
+};
+
+// MS-SSIM scales 2 .. 4 of one plane from scale 1, each the 2x2 means of the one before (xPixelOpsSTD.cpp:50-67)
+struct SsimPyrJob
+{
+  const void* src;             // scale 1, pitch W
+  void*       dst[3];          // scales 2, 3, 4, null where not needed
+  int32_t     W, H;            // of scale 1
+  int32_t     esz, pad_;
 };
 
 // windows from moments, ordered row sums (xSSIM.cpp:353-369), for up to 6 (pair, component) jobs
@@ -91,14 +109,33 @@ struct SsimPoolJob
   int32_t         calc_l;
   int32_t         wide;        // window sums can exceed 32 bits (bit depth > 12)
   int32_t         pad_;
-  double*         row_sum;     // [ny]
-  double*         win;         // scratch window values [ceil(ny / 32)][nx][32] (pool_win_elems)
+  double*         win;         // window values [ceil(ny / 32)][nx][32] (pool_win_elems)
 };
 
-struct SsimPoolArgs
+// The launches of one pair's block SSIM family (add_ssim_jobs): windows from the search's moments, windows
+// from the pictures at scale 0 and at the smaller scales, the scales between, row sums of all windows.
+constexpr int kMaxPoolJobs = 6, kMaxImgJobs0 = 12, kMaxImgJobsN = 36, kMaxPyrJobs = 12, kMaxRowJobs = kMaxPoolJobs + kMaxImgJobs0 + kMaxImgJobsN;
+struct SsimRowJob
 {
-  int32_t     njobs;
-  SsimPoolJob job[9];
+  const double* win;           // [ceil(ny / 32)][nx][32]
+  double*       row_sum;       // [ny]
+  int32_t       nx, ny;
+};
+template <typename J, int N> struct JobArgs { J job[N]; };   // by-value form of a launch's jobs
+struct SsimJobs
+{
+  int32_t npool = 0, nimg0 = 0, nimgn = 0, npyr = 0, nrows = 0;
+  JobArgs<SsimPoolJob, kMaxPoolJobs> pool;
+  JobArgs<SsimImgJob, kMaxImgJobs0>  img0;
+  JobArgs<SsimImgJob, kMaxImgJobsN>  imgn;
+  JobArgs<SsimPyrJob, kMaxPyrJobs>   pyr;
+  JobArgs<SsimRowJob, kMaxRowJobs>   rows;
+};
+// Largest window grid / plane of the jobs of each launch, over every pair that shares it
+struct SsimDims
+{
+  int pool_nx = 0, pool_ny = 0, img0_nx = 0, img0_ny = 0, imgn_nx = 0, imgn_ny = 0, pyr_w = 0, pyr_h = 0, rows_ny = 0;
+  void add(const SsimJobs& q);
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -166,6 +203,25 @@ struct FinalizeArgs
   PairOut*        out;
 };
 
+// The pictures, buffers and sizes of one pair's block SSIM family
+struct SsimPairArgs
+{
+  Img      in0, in1, scp0, scp1;   // scp: 4:4:4, where IV-MS-SSIM needs them
+  uint32_t mask;
+  int32_t  W, H, esz, bitdepth;
+  uint32_t clip;
+  int32_t  ns;                     // MS-SSIM scales
+  int32_t  nx[5], ny[5];
+  double   C1, C2;
+  int32_t  use_ws;                 // ERP row weights of IV-SSIM
+  Moments  mom[2];                 // of the search: (In0, SCP1), (In1, SCP0)
+  double*  rowsum;                 // [kMaxSsimSlots][3][ny[0]]
+  double*  win;                    // ssim_win_elems doubles
+  char*    pyr;                    // scales 1 .. ns - 1 of In0, In1, SCP0, SCP1
+};
+size_t ssim_win_elems(uint32_t mask, int ns, const int32_t nx[5], const int32_t ny[5]);
+void   add_ssim_jobs(const SsimPairArgs& p, SsimJobs& q, FinalizeArgs& fa);
+
 // one (pair, chain) CTA of the multi-pair finalize; chain == nchains of the pair is its exact CPS sums
 struct FinJob
 {
@@ -177,9 +233,21 @@ constexpr size_t kFinalizeMaxSmem = 200 * 1024;
 template <typename T> cudaError_t launch_prepass(const PrepassArgs& a, cudaStream_t s);
 cudaError_t launch_reduce(const ReduceArgs& a, cudaStream_t s);
 template <typename T> cudaError_t launch_cps(const CpsArgs& a, int R, cudaStream_t s);
-template <typename T> cudaError_t launch_ssim_moments(const SsimMomArgs& a, cudaStream_t s);
-cudaError_t launch_ssim_pool(const SsimPoolArgs& a, cudaStream_t s);
-cudaError_t launch_ssim_rows(const SsimPoolArgs& a, cudaStream_t s);   // row sums of ready window values
+// Block SSIM launches of one pair (jobs by value) or of many (job tables in device memory, one after the
+// other: pool, img0, imgn, pyr, rows with n entries each)
+cudaError_t launch_ssim_jobs(const SsimJobs& q, cudaStream_t s, bool rows_only);
+struct SsimTables
+{
+  const SsimPoolJob* pool = nullptr;
+  const SsimImgJob*  img0 = nullptr;
+  const SsimImgJob*  imgn = nullptr;
+  const SsimPyrJob*  pyr = nullptr;
+  const SsimRowJob*  rows = nullptr;
+  int npool = 0, nimg0 = 0, nimgn = 0, npyr = 0, nrows = 0;
+  SsimDims dims;
+};
+cudaError_t launch_ssim_tables(const SsimTables& t, cudaStream_t s, bool rows_only);
+cudaError_t launch_ssim_rows(const JobArgs<SsimRowJob, kMaxRowJobs>& a, int njobs, cudaStream_t s);   // row sums of ready window values
 // SSIM windows of one option set for up to kGenMaxJobs jobs: mode QMIV_SSM_*, window N, stride S,
 // border QMIV_BRD_* (regular modes)
 cudaError_t launch_ssim_gen(SsimGenArgs& a, int mode, int N, int S, int border, cudaStream_t s);
@@ -193,10 +261,7 @@ size_t      finalize_smem(const FinalizeArgs& a);
 // multi-pair forms: argument blocks in device memory, one launch for every pair of a batch
 template <typename T> cudaError_t launch_prepass_multi(const PrepassArgs* d_jobs, int njobs, int max_rows, cudaStream_t s);
 cudaError_t launch_reduce_multi(const ReduceArgs* d_jobs, int njobs, cudaStream_t s);
-template <typename T>
-cudaError_t launch_ssim_moments_multi(const SsimMomArgs* d_jobs, int njobs, int max_nbx, int max_nby, cudaStream_t s);
-cudaError_t launch_ssim_pool_multi(const SsimPoolJob* d_jobs, int njobs, int max_nx, int max_ny, cudaStream_t s);
-size_t      pool_win_elems(int nx, int ny);   // doubles of SsimPoolJob::win
+size_t      pool_win_elems(int nx, int ny);   // doubles of the windows of nx x ny
 // 16-byte alignment of the moment rows and the scratch, which the pooling kernels copy with cp.async
 bool        pool_job_aligned(const SsimPoolJob& J);
 cudaError_t launch_finalize_multi(const FinalizeArgs* d_pairs, const FinJob* d_jobs, int njobs, size_t smem, cudaStream_t s);
