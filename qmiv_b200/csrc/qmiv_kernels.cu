@@ -258,8 +258,13 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a, int chain, 
   const int len = ch.kind == kChainSsim ? a.slot[ch.a].ny : a.H;
   double* vals = stage;
   double* wts = stage + len;
+  __shared__ unsigned long long top[2];                      // largest term of the values and of the weights
+  __shared__ double wtotal;
+  if(threadIdx.x < 2) { top[threadIdx.x] = 0ull; }
+  __syncthreads();
   // eight rows per thread and pass with their loads issued together (one round trip per pass)
   constexpr int U = 8;
+  unsigned long long tv = 0ull, tw = 0ull;
   for(int y0 = threadIdx.x; y0 < len; y0 += 256 * U)
   {
     double v[U], w[U];
@@ -275,21 +280,24 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a, int chain, 
     {
       const int y = y0 + u * 256;
       if(y < len) { vals[y] = v[u]; if(wsum) { wts[y] = w[u]; } }
+      tv = max(tv, term_bits(v[u])); tw = max(tw, term_bits(w[u]));
     }
+  }
+  #pragma unroll
+  for(int o2 = 16; o2 > 0; o2 >>= 1) { tv = max(tv, __shfl_xor_sync(kFull, tv, o2)); tw = max(tw, __shfl_xor_sync(kFull, tw, o2)); }
+  if((threadIdx.x & 31) == 0) { atomicMax(&top[0], tv); atomicMax(&top[1], tw); }
+  __syncthreads();
+  // thread 0 sums the values; a weighted chain's weights are summed beside it by the second warp
+  Kbns sum;
+  if(threadIdx.x == 0) { chain_sum(sum, vals, len, top[0]); }
+  if(threadIdx.x == 32 && wsum)
+  {
+    Kbns wk;
+    chain_sum(wk, wts, len, top[1]);
+    wtotal = wk.result();
   }
   __syncthreads();
   if(threadIdx.x != 0) { return; }
-  Kbns sum, wk;
-  int y = 0;
-  for(; y + 8 <= len; y += 8)
-  {
-    double v[8], w[8];
-    #pragma unroll
-    for(int u = 0; u < 8; u++) { v[u] = vals[y + u]; w[u] = wsum ? wts[y + u] : 0.0; }
-    #pragma unroll
-    for(int u = 0; u < 8; u++) { sum.add(v[u]); if(wsum) { wk.add(w[u]); } }
-  }
-  for(; y < len; y++) { sum.add(vals[y]); if(wsum) { wk.add(wts[y]); } }
   if(ch.kind == kChainWsPsnr) { o->ws_ssd[ch.a] = sum.result(); }
   else if(ch.kind == kChainIvPsnr) { o->cps_ws[ch.a][ch.b] = sum.result(); }
   else
@@ -299,7 +307,7 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a, int chain, 
     double r;
     if(wsum)
     {
-      const double corr = ddiv(wk.result(), (double)sl.ny);
+      const double corr = ddiv(wtotal, (double)sl.ny);
       r = ddiv(sum.result(), dmul(active, corr));
     }
     else { r = ddiv(sum.result(), active); }

@@ -925,7 +925,7 @@ constexpr int kMaskFinChunk = 4096;
 __device__ __forceinline__ void mask_finalize_body(const MaskArgs& a, int chain)
 {
   __shared__ double vals[kMaskFinChunk];
-  __shared__ unsigned long long tot;
+  __shared__ unsigned long long tot, top;
   const int k = chain;
   if(k < 3 && !a.ws) { return; }                              // uniform over the CTA
   MaskOut* o = a.out;
@@ -941,6 +941,9 @@ __device__ __forceinline__ void mask_finalize_body(const MaskArgs& a, int chain)
   {
     const int n = min(kMaskFinChunk, H - base);
     __syncthreads();                                          // the previous chunk has been summed
+    if(threadIdx.x == 0) { top = 0ull; }
+    __syncthreads();
+    unsigned long long tv = 0ull;
     constexpr int U = kMaskFinChunk / 256;                    // a thread's loads all in flight at once
     uint64_t v[U];
     double w[U];
@@ -955,14 +958,18 @@ __device__ __forceinline__ void mask_finalize_body(const MaskArgs& a, int chain)
     for(int u = 0; u < U; u++)
     {
       const int i = threadIdx.x + u * 256;
-      if(i < n) { loc += v[u]; vals[i] = a.ws ? dmul((double)v[u], w[u]) : 0.0; }
+      if(i < n)
+      {
+        loc += v[u];
+        vals[i] = a.ws ? dmul((double)v[u], w[u]) : 0.0;
+        tv = max(tv, term_bits(vals[i]));
+      }
     }
+    #pragma unroll
+    for(int o2 = 16; o2 > 0; o2 >>= 1) { tv = max(tv, __shfl_xor_sync(0xffffffffu, tv, o2)); }
+    if((threadIdx.x & 31) == 0) { atomicMax(&top, tv); }
     __syncthreads();
-    if(threadIdx.x == 0 && a.ws)
-    {
-      #pragma unroll 8
-      for(int i = 0; i < n; i++) { s.add(vals[i]); }
-    }
+    if(threadIdx.x == 0 && a.ws) { chain_sum(s, vals, n, top); }
   }
   loc = warp_sum_u64(loc);                                    // exact: integer sum in any order
   if((threadIdx.x & 31) == 0) { atomicAdd(&tot, loc); }
