@@ -478,8 +478,10 @@ __device__ __forceinline__ void ssim_rows_body(const SsimRowJob& J, int band)
     // nothing and are not written
     if(cols == kRowCols && __all_sync(0xffffffffu, band * 32 + lane >= J.ny || row.s >= 2.0 * (kRowCols + 1)))
     {
+      double v[kRowCols];
       #pragma unroll
-      for(int x = 0; x < kRowCols; x++) { row.add_small(b[x][lane]); }
+      for(int x = 0; x < kRowCols; x++) { v[x] = b[x][lane]; }
+      row.add_small(v);
     }
     else if(cols == kRowCols)
     {
