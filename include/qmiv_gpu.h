@@ -270,7 +270,7 @@ QMIV_API qmiv_status qmiv_calc_stream(qmiv_calc calc, void** cuda_stream);
    until the result is in `out`; it synchronises that stream and copies from pageable host memory, so
    it must not be called on a stream that is being captured into a CUDA graph. It calls no
    cudaMalloc, cudaFree or other allocating routine: its scratch is one fixed file-scope device array
-   (about 350 KB per GPU), which limits the picture height to QMIV_STATIC_MAX_HEIGHT rows; taller
+   (about 250 KB per GPU), which limits the picture height to QMIV_STATIC_MAX_HEIGHT rows; taller
    pictures are rejected with QMIV_ERR_UNSUPPORTED. The array comes with the library's device code:
    with CUDA's lazy module loading (the default) it is placed on a GPU at this entry point's first
    call there, and it stays until the process exits, so a caller that may not allocate after

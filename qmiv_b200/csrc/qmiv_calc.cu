@@ -180,14 +180,14 @@ qmiv_status PairPipeline::prepare(uint32_t mask, bool want_scp, bool host_frames
 {
   const Shape& S = shape_;
   const size_t rows_total = (size_t)S.H + 2 * (size_t)S.ch;
-  QMIV_TRY(row_sd_.ensure(ctx_, rows_total * sizeof(int64_t)));
   QMIV_TRY(row_ssd_.ensure(ctx_, rows_total * sizeof(uint64_t)));
-  QMIV_TRY(out_.ensure(ctx_, sizeof(PairOut)));
   const bool need_scp = need_scp_for(mask, want_scp);
   const bool need_search = need_scp || (mask & (QMIV_IVPSNR | QMIV_IVSSIM));
   const bool need_ssim = mask & (QMIV_SSIM | QMIV_MSSSIM | QMIV_IVSSIM | QMIV_IVMSSSIM);
   const bool need_ms = mask & (QMIV_MSSSIM | QMIV_IVMSSSIM);
-  if(need_search) { QMIV_TRY(cps_rows_.ensure(ctx_, (size_t)2 * S.H * 3 * sizeof(uint32_t))); }
+  // the result block and, behind it, the search's row sums: one memset clears both
+  QMIV_TRY(out_.ensure(ctx_, kRowsOffset + (need_search ? (size_t)2 * S.H * 3 * sizeof(uint32_t) : 0)));
+  if(need_search) { has_rows_ = true; }
   if(need_scp) { QMIV_TRY(scp_.ensure(ctx_, (size_t)2 * 3 * S.W * S.H * S.esz)); }
   // moments of the two IV-SSIM directions, written by the search
   if((mask & QMIV_IVSSIM) && !gen_) { QMIV_TRY(mom_.ensure(ctx_, (size_t)2 * mom_slot_elems() * sizeof(uint32_t))); }
@@ -317,30 +317,25 @@ qmiv_status PairPipeline::enqueue_t(const Img& in0, const Img& in1, uint32_t mas
   const uint32_t clip = prm_.invalid_pel_action == QMIV_PEL_CNCL ? (uint32_t)S.maxv : 0xffffu;
   PairOut* dout = out_.as<PairOut>();
 
-  QMIV_CUDA(cudaMemsetAsync(dout, 0, sizeof(PairOut), s));
-  if(need_search) { QMIV_CUDA(cudaMemsetAsync(cps_rows_.p, 0, (size_t)2 * S.H * 3 * sizeof(uint32_t), s)); }
+  QMIV_CUDA(cudaMemsetAsync(dout, 0, need_search ? kRowsOffset + (size_t)2 * S.H * 3 * sizeof(uint32_t) : sizeof(PairOut), s));
 
-  // 1. prepass + reduce (GCD)
+  // 1. prepass (totals, GCD)
   PrepassArgs pa{};
   pa.in0 = in0; pa.in1 = in1;
   for(int c = 0; c < 3; c++) { pa.rows[c] = (int32_t)S.plane_rows(c); pa.cols[c] = (int32_t)S.plane_cols(c); }
-  pa.clip = clip; pa.row_sd = row_sd_.as<int64_t>(); pa.row_ssd = row_ssd_.as<uint64_t>(); pa.out = dout;
-  { const int t = prof_begin(s); QMIV_CUDA(launch_prepass<T>(pa, s)); prof_end(s, QMIV_STAGE_PREPASS, t); }
-
-  ReduceArgs ra{};
-  for(int c = 0; c < 3; c++) { ra.rows[c] = pa.rows[c]; ra.mult[c] = c ? (1 << (S.sx + S.sy)) : 1; }
-  ra.area = (int64_t)S.W * S.H; ra.maxv = S.maxv;
-  for(int c = 0; c < 4; c++) { ra.maxdiff[c] = maxdiff_[c]; }
-  ra.need_gcd = need_search || want_gcd; ra.fp32_ok = fp32_ok_; ra.clip_on = prm_.invalid_pel_action == QMIV_PEL_CNCL;
+  pa.clip = clip; pa.row_ssd = row_ssd_.as<uint64_t>(); pa.out = dout;
+  for(int c = 0; c < 3; c++) { pa.mult[c] = c ? (1 << (S.sx + S.sy)) : 1; }
+  pa.area = (int64_t)S.W * S.H; pa.maxv = S.maxv;
+  for(int c = 0; c < 4; c++) { pa.maxdiff[c] = maxdiff_[c]; }
+  pa.need_gcd = need_search || want_gcd; pa.fp32_ok = fp32_ok_; pa.clip_on = prm_.invalid_pel_action == QMIV_PEL_CNCL;
   if(gcd_override_on_)
   {
     int32_t mag[4];
-    for(int c = 0; c < 4; c++) { ra.gcd_override[c] = gcd_override_[c]; mag[c] = gcd_override_[c] < 0 ? -gcd_override_[c] : gcd_override_[c]; }
-    ra.gcd_override_on = 1;
-    ra.fp32_ok = cps_key_exact(R_, S.sx, S.sy, S.maxv, prm_.cws, mag);
+    for(int c = 0; c < 4; c++) { pa.gcd_override[c] = gcd_override_[c]; mag[c] = gcd_override_[c] < 0 ? -gcd_override_[c] : gcd_override_[c]; }
+    pa.gcd_override_on = 1;
+    pa.fp32_ok = cps_key_exact(R_, S.sx, S.sy, S.maxv, prm_.cws, mag);
   }
-  ra.row_sd = pa.row_sd; ra.row_ssd = pa.row_ssd; ra.out = dout;
-  { const int t = prof_begin(s); QMIV_CUDA(launch_reduce(ra, s)); prof_end(s, QMIV_STAGE_REDUCE, t); }
+  { const int t = prof_begin(s); QMIV_CUDA(launch_prepass<T>(pa, s)); prof_end(s, QMIV_STAGE_PREPASS, t); }
 
   // 2. CPS search, both directions, SCP pictures when needed
   if(need_search)
@@ -349,7 +344,7 @@ qmiv_status PairPipeline::enqueue_t(const Img& in0, const Img& in1, uint32_t mas
     ca.in0 = in0; ca.in1 = in1; ca.W = S.W; ca.H = S.H; ca.maxv = S.maxv; ca.clip = clip;
     for(int c = 0; c < 3; c++) { ca.wi[c] = prm_.cws[c]; ca.wf[c] = (float)prm_.cws[c]; }
     for(int c = 0; c < 3; c++) { ca.gmax[c] = gcd_override_on_ ? gcd_override_[c] : maxdiff_[c]; }
-    ca.gcd_src = dout; ca.rows = cps_rows_.as<uint32_t>();
+    ca.gcd_src = dout; ca.rows = rows_device();
     ca.scp0 = need_scp ? const_cast<void*>(scp(0)) : nullptr;
     ca.scp1 = need_scp ? const_cast<void*>(scp(1)) : nullptr;
     if((mask & QMIV_IVSSIM) && !gen_) { ca.mom[0] = mom_at(0, 0); ca.mom[1] = mom_at(1, 0); }  // (In0, SCP1), (In1, SCP0)
@@ -397,7 +392,7 @@ qmiv_status PairPipeline::enqueue_t(const Img& in0, const Img& in1, uint32_t mas
   fa.row_ssd = row_ssd_.as<uint64_t>();
   fa.ws = prm_.erp ? ws_.as<double>() : nullptr;
   fa.do_wspsnr = (mask & QMIV_WSPSNR) ? 1 : 0;
-  fa.cps_rows = need_search ? cps_rows_.as<uint32_t>() : nullptr;
+  fa.cps_rows = need_search ? rows_device() : nullptr;
   fa.out = dout;
   { const int t = prof_begin(s); QMIV_CUDA(launch_finalize(fa, s)); prof_end(s, QMIV_STAGE_FINALIZE, t); }
   { const int t = prof_begin(s); QMIV_CUDA(cudaMemcpyAsync(h_out, dout, sizeof(PairOut), cudaMemcpyDeviceToHost, s)); prof_end(s, QMIV_STAGE_D2H, t); }

@@ -167,7 +167,8 @@ struct PairOut
   int32_t  flags;            // bit0: frame0 invalid, bit1: frame1 invalid, bit2: integer CPS path,
                              // bit3: a CPS tile load did not complete (bounded wait ran out)
   uint32_t max_sample[2];
-  int64_t  sd[3];            // 4:4:4 totals of In1 - In0
+  uint32_t done;             // CTAs of the prepass that have added their rows
+  int64_t  sd[3];            // 4:4:4 totals of In1 - In0 (raw sums while the prepass runs)
   uint64_t ssd[3];           // 4:4:4 totals
   double   ws_ssd[3];        // KBNS over rows of rowSSD*w[y] (WS-PSNR, before correction)
   uint64_t cps_sum[2][3];    // sum over rows of sign-extended 32-bit row sums, [R2T, T2R]

@@ -2,8 +2,7 @@
 // every stage of the pipeline one launch for all pairs.
 //
 //   descriptors   one host-to-device copy of every pair's argument blocks (tensor maps included)
-//   prepass       one launch per sample size, a CTA row per pair          (k_prepass_multi)
-//   reduce        one CTA per pair                                        (k_reduce_multi)
+//   prepass       one launch per sample size, a CTA row per pair, totals and GCD by its last (k_prepass_multi)
 //   CPS           one persistent launch per (R, sample size, tile height) over a work list of the
 //                 tiles of all its pairs                                   (k_cps_multi)
 //   SSIM          windows of all pairs at scale 0, the smaller scales, their windows, every window row
@@ -294,7 +293,6 @@ qmiv_status Engine::submit(const qmiv_pair_desc* pairs, int32_t n)
     const PairKind& K = *kind[i];
     const Shape& S = K.S;
     const size_t rows_total = (size_t)S.H + 2 * (size_t)S.ch;
-    p.row_sd = take(rows_total * sizeof(int64_t));
     p.row_ssd = take(rows_total * sizeof(uint64_t));
     if(p.need_scp) { p.scp = take((size_t)2 * 3 * S.W * S.H * S.esz); }
     if(p.need_ssim)
@@ -598,7 +596,6 @@ qmiv_status Engine::build_tables(int first, int n, const std::vector<PairKind*>&
   auto place = [&](size_t bytes, size_t align) { off = align_sz(off, align); const size_t o = off; off += bytes; return o; };
   T.prepass_off[0] = place(sizeof(PrepassArgs) * T.prepass_idx[0].size(), 64);
   T.prepass_off[1] = place(sizeof(PrepassArgs) * T.prepass_idx[1].size(), 64);
-  T.reduce_off = place(sizeof(ReduceArgs) * (size_t)n, 64);
   size_t ncps = 0;
   for(auto& g : T.cps_groups) { ncps += g.second.size(); }
   T.cps_off = place(cps_desc_bytes() * ncps, 64);
@@ -630,7 +627,7 @@ void Engine::fill_tables(int n, const std::vector<PairKind*>& kind, const std::v
                          const std::vector<Img>& in1, char* dbase, Tables& T, char* h, char* d)
 {
   const int first = T.first;
-  // prepass + reduce
+  // prepass
   for(int g = 0; g < 2; g++)
   {
     PrepassArgs* pa = reinterpret_cast<PrepassArgs*>(h + T.prepass_off[g]);
@@ -643,26 +640,15 @@ void Engine::fill_tables(int n, const std::vector<PairKind*>& kind, const std::v
       a.in0 = in0[i]; a.in1 = in1[i];
       for(int c = 0; c < 3; c++) { a.rows[c] = (int32_t)K.S.plane_rows(c); a.cols[c] = (int32_t)K.S.plane_cols(c); }
       a.clip = clip_of(K);
-      a.row_sd = reinterpret_cast<int64_t*>(dbase + p.row_sd);
       a.row_ssd = reinterpret_cast<uint64_t*>(dbase + p.row_ssd);
       a.out = reinterpret_cast<PairOut*>(dbase + p.out);
+      for(int c = 0; c < 3; c++) { a.mult[c] = c ? (1 << (K.S.sx + K.S.sy)) : 1; }
+      a.area = (int64_t)K.S.W * K.S.H; a.maxv = K.S.maxv;
+      for(int c = 0; c < 4; c++) { a.maxdiff[c] = K.maxdiff[c]; }
+      a.need_gcd = p.need_search ? 1 : 0;
+      a.fp32_ok = K.fp32_ok ? 1 : 0;
+      a.clip_on = prm_.invalid_pel_action == QMIV_PEL_CNCL;
     }
-  }
-  ReduceArgs* ra = reinterpret_cast<ReduceArgs*>(h + T.reduce_off);
-  for(int i = first; i < first + n; i++)
-  {
-    const PairKind& K = *kind[i];
-    const PairSlot& p = slots_[i];
-    ReduceArgs& a = ra[i - first];
-    for(int c = 0; c < 3; c++) { a.rows[c] = (int32_t)K.S.plane_rows(c); a.mult[c] = c ? (1 << (K.S.sx + K.S.sy)) : 1; }
-    a.area = (int64_t)K.S.W * K.S.H; a.maxv = K.S.maxv;
-    for(int c = 0; c < 4; c++) { a.maxdiff[c] = K.maxdiff[c]; }
-    a.need_gcd = p.need_search ? 1 : 0;
-    a.fp32_ok = K.fp32_ok ? 1 : 0;
-    a.clip_on = prm_.invalid_pel_action == QMIV_PEL_CNCL;
-    a.row_sd = reinterpret_cast<int64_t*>(dbase + p.row_sd);
-    a.row_ssd = reinterpret_cast<uint64_t*>(dbase + p.row_ssd);
-    a.out = reinterpret_cast<PairOut*>(dbase + p.out);
   }
   // CPS work lists
   {
@@ -768,7 +754,6 @@ void Engine::fill_tables(int n, const std::vector<PairKind*>& kind, const std::v
   T.d_finjobs = reinterpret_cast<const FinJob*>(d + T.finjob_off);
   T.d_prepass[0] = reinterpret_cast<const PrepassArgs*>(d + T.prepass_off[0]);
   T.d_prepass[1] = reinterpret_cast<const PrepassArgs*>(d + T.prepass_off[1]);
-  T.d_reduce = reinterpret_cast<const ReduceArgs*>(d + T.reduce_off);
 }
 
 qmiv_status Engine::launch_all(const Tables& T, cudaStream_t s)
@@ -778,11 +763,6 @@ qmiv_status Engine::launch_all(const Tables& T, cudaStream_t s)
     QMIV_CUDA(launch_prepass_multi<uint8_t>(T.d_prepass[0], (int)T.prepass_idx[0].size(), T.prepass_max_rows[0], s));
     QMIV_CUDA(launch_prepass_multi<uint16_t>(T.d_prepass[1], (int)T.prepass_idx[1].size(), T.prepass_max_rows[1], s));
     prof_end(s, QMIV_STAGE_PREPASS, t);
-  }
-  {
-    const int t = prof_begin(s);
-    QMIV_CUDA(launch_reduce_multi(T.d_reduce, T.n, s));
-    prof_end(s, QMIV_STAGE_REDUCE, t);
   }
   for(const CpsLaunch& L : T.cps_launch)
   {

@@ -40,7 +40,7 @@ struct PairSlot
 {
   uint32_t mask = 0;
   bool     need_scp = false, need_search = false, need_ssim = false, need_ms = false, host = false;
-  size_t   out = 0, cps_rows = 0, row_sd = 0, row_ssd = 0, scp = 0, mom = 0, mom_slot = 0, rowsum = 0, win = 0;
+  size_t   out = 0, cps_rows = 0, row_ssd = 0, scp = 0, mom = 0, mom_slot = 0, rowsum = 0, win = 0;
   size_t   pyr = 0, pyr_lv = 0, staging = 0;
 };
 
@@ -67,7 +67,7 @@ struct Tables
   int    first = 0;                 // global index of the set's first pair
   std::vector<int> prepass_idx[2];
   int    prepass_max_rows[2] = { 0, 0 };
-  size_t prepass_off[2] = { 0, 0 }, reduce_off = 0, cps_off = 0, prefix_off = 0, fin_off = 0;
+  size_t prepass_off[2] = { 0, 0 }, cps_off = 0, prefix_off = 0, fin_off = 0;
   size_t pool_off = 0, img0_off = 0, imgn_off = 0, pyr_off = 0, rows_off = 0, finjob_off = 0;
   std::map<CpsGroupKey, std::vector<int>> cps_groups;
   std::vector<CpsLaunch> cps_launch;
@@ -75,7 +75,6 @@ struct Tables
   int    fin_jobs = 0;
   size_t fin_smem = 0;
   const PrepassArgs*  d_prepass[2] = { nullptr, nullptr };
-  const ReduceArgs*   d_reduce = nullptr;
   const FinalizeArgs* d_fin = nullptr;
   const FinJob*       d_finjobs = nullptr;
 };

@@ -161,7 +161,7 @@ public:
   FinishInfo finish_info(uint32_t mask) const;
   // SCP planes (T samples, planar 3 x W*H) of the last run, or null
   const void* scp(int which) const;
-  const uint32_t* cps_rows() const { return cps_rows_.as<uint32_t>(); }
+  const uint32_t* cps_rows() const { return has_rows_ ? rows_device() : nullptr; }
   const double* ws_device() const { return ws_.as<double>(); }   // ERP row weights, after prepare()
   double ws_corr() const { return ws_corr_; }
   const int32_t* maxdiff() const { return maxdiff_; }
@@ -226,7 +226,11 @@ private:
     return 3 * 5 * nby * ((nbx + 7) & ~(size_t)7);
   }
 
-  DevMem row_sd_, row_ssd_, cps_rows_, out_, ws_, scp_, pyr_, mom_, rowsum_, win_, staging_;
+  // the search's 32-bit row sums lie behind the result block
+  static constexpr size_t kRowsOffset = (sizeof(PairOut) + 255) & ~(size_t)255;
+  uint32_t* rows_device() const { return reinterpret_cast<uint32_t*>(out_.as<char>() + kRowsOffset); }
+  bool   has_rows_ = false;
+  DevMem row_ssd_, out_, ws_, scp_, pyr_, mom_, rowsum_, win_, staging_;
   PairOut* h_out = nullptr;
   bool ws_uploaded_ = false;
   bool gcd_override_on_ = false;

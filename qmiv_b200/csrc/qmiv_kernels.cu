@@ -2,9 +2,9 @@
 //
 // Pipeline of one frame pair (the reference runs the same steps per frame on the CPU,
 // apps/QMIV/src/xAppQMIV.cpp:761-827):
-//   k_prepass   per raw row: SD(In1-In0), SSD, max sample        (HBM bound, reads both frames once)
-//   k_reduce    totals, GCD, exactness of the fp32 search path   (one CTA)
-//   k_cps       (qmiv_cps.cu) corresponding-pixel-shift search, both directions in one pass;
+//   k_prepass   SD(In1-In0), SSD per raw row, max sample (HBM bound, reads both frames once); its last
+//               CTA: totals, GCD, exactness of the key search path
+//   k_cps       (qmiv_cps.cu, qmiv_cps420.cu) corresponding-pixel-shift search, both directions in one pass;
 //               per-row SSE into 32-bit lanes, the IV-SSIM sub-block moments of (test, SCP) and,
 //               when IV-MS-SSIM or the caller needs them, the shift-compensated pictures
 //   k_ssim_*    (qmiv_ssim.cu) block SSIM from exact integer moments, FP64 windows, row sums
@@ -21,13 +21,15 @@ constexpr unsigned kFull = 0xffffffffu;
 // =============================================================================================
 // prepass
 // =============================================================================================
+// A warp takes one raw row. Its sums join the picture's by way of the CTA (eight rows, six additions to the
+// result block), and the CTA that adds last turns the totals into the GCD (xGlobClrDiff.cpp:70-103) and the
+// path flags: a launch of its own for that took 7 us of a one-pair call, most of it latency.
 template <typename T>
-__device__ __forceinline__ void prepass_body(const PrepassArgs& a, int warp)
+__device__ __forceinline__ void prepass_row(const PrepassArgs& a, int warp, int lane, int& c, int64_t& sd_out, uint64_t& ssd_out, uint32_t& m0_out,
+                                            uint32_t& m1_out)
 {
-  const int lane  = threadIdx.x & 31;
-  const int total = a.rows[0] + a.rows[1] + a.rows[2];
-  if(warp >= total) { return; }
-  int c = 0, r = warp;
+  int r = warp;
+  c = 0;
   if(r >= a.rows[0]) { r -= a.rows[0]; c = 1; if(r >= a.rows[1]) { r -= a.rows[1]; c = 2; } }
   const T* p0 = static_cast<const T*>(a.in0.p[c]) + (size_t)r * a.in0.pitch[c];
   const T* p1 = static_cast<const T*>(a.in1.p[c]) + (size_t)r * a.in1.pitch[c];
@@ -80,28 +82,73 @@ __device__ __forceinline__ void prepass_body(const PrepassArgs& a, int warp)
     sd  += __shfl_xor_sync(kFull, sd, o);
     ssd += __shfl_xor_sync(kFull, ssd, o);
   }
-  m0 = __reduce_max_sync(kFull, m0);
-  m1 = __reduce_max_sync(kFull, m1);
-  if(lane == 0)
+  m0_out = __reduce_max_sync(kFull, m0);
+  m1_out = __reduce_max_sync(kFull, m1);
+  sd_out = sd;
+  ssd_out = ssd;
+  if(lane == 0) { a.row_ssd[warp] = ssd; }
+}
+
+__device__ __forceinline__ void prepass_totals(const PrepassArgs& a);
+
+template <typename T>
+__device__ __forceinline__ void prepass_body(const PrepassArgs& a, int block)
+{
+  __shared__ int64_t  s_sd[8];
+  __shared__ uint64_t s_ssd[8];
+  __shared__ uint32_t s_m[2][8];
+  __shared__ int32_t  s_c[8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warp = block * 8 + wid;
+  const int total = a.rows[0] + a.rows[1] + a.rows[2];
+  if(block * 8 >= total) { return; }                       // uniform: not a CTA of this pair
+  int c = -1;
+  int64_t sd = 0;
+  uint64_t ssd = 0;
+  uint32_t m0 = 0, m1 = 0;
+  if(warp < total) { prepass_row<T>(a, warp, lane, c, sd, ssd, m0, m1); }
+  if(lane == 0) { s_sd[wid] = sd; s_ssd[wid] = ssd; s_m[0][wid] = m0; s_m[1][wid] = m1; s_c[wid] = c; }
+  __syncthreads();
+  if(threadIdx.x >= 32) { return; }
+  PairOut* o = a.out;
+  if(lane < 6)
   {
-    a.row_sd[warp]  = sd;
-    a.row_ssd[warp] = ssd;
-    atomicMax(&a.out->max_sample[0], m0);
-    atomicMax(&a.out->max_sample[1], m1);
+    const int k = lane % 3;
+    unsigned long long v = 0;
+    bool any = false;
+    #pragma unroll
+    for(int w = 0; w < 8; w++)
+    {
+      if(s_c[w] == k) { v += lane < 3 ? (unsigned long long)s_sd[w] : (unsigned long long)s_ssd[w]; any = true; }
+    }
+    if(any) { atomicAdd(lane < 3 ? reinterpret_cast<unsigned long long*>(&o->sd[k]) : reinterpret_cast<unsigned long long*>(&o->ssd[k]), v); }
+  }
+  else if(lane < 8)
+  {
+    uint32_t m = 0;
+    #pragma unroll
+    for(int w = 0; w < 8; w++) { m = max(m, s_m[lane - 6][w]); }
+    atomicMax(&o->max_sample[lane - 6], m);
+  }
+  __threadfence();                                          // the additions before the count
+  __syncwarp();
+  if(lane == 0 && atomicAdd(&o->done, 1u) == (uint32_t)((total + 7) / 8) - 1u)
+  {
+    __threadfence();
+    prepass_totals(a);
   }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_prepass(const __grid_constant__ PrepassArgs a)
 {
-  prepass_body<T>(a, (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5));
+  prepass_body<T>(a, (int)blockIdx.x);
 }
 
 // one job (frame pair) per blockIdx.y
 template <typename T>
 __global__ void __launch_bounds__(256) k_prepass_multi(const PrepassArgs* __restrict__ jobs)
 {
-  prepass_body<T>(jobs[blockIdx.y], (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5));
+  prepass_body<T>(jobs[blockIdx.y], (int)blockIdx.x);
 }
 
 template <typename T>
@@ -125,71 +172,30 @@ cudaError_t launch_prepass_multi(const PrepassArgs* d_jobs, int njobs, int max_r
 template cudaError_t launch_prepass_multi<uint8_t>(const PrepassArgs*, int, int, cudaStream_t);
 template cudaError_t launch_prepass_multi<uint16_t>(const PrepassArgs*, int, int, cudaStream_t);
 
-// =============================================================================================
-// reduce: totals and GCD (libs/pmbb-ivqm/src/xGlobClrDiff.cpp:70-103)
-// =============================================================================================
-__device__ __forceinline__ void reduce_body(const ReduceArgs& a)
+// Totals, GCD and path flags, by one thread of the last CTA (libs/pmbb-ivqm/src/xGlobClrDiff.cpp:70-103).
+__device__ __forceinline__ void prepass_totals(const PrepassArgs& a)
 {
-  __shared__ int64_t  s_sd[3][32];
-  __shared__ uint64_t s_ssd[3][32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int off = 0;
+  PairOut* o = a.out;
+  const double area = (double)a.area;
+  int64_t sd[4] = { 0, 0, 0, 0 };
   for(int c = 0; c < 3; c++)
   {
-    int64_t sd = 0; uint64_t ssd = 0;
-    for(int r = threadIdx.x; r < a.rows[c]; r += blockDim.x) { sd += a.row_sd[off + r]; ssd += a.row_ssd[off + r]; }
-    #pragma unroll
-    for(int o = 16; o > 0; o >>= 1) { sd += __shfl_xor_sync(kFull, sd, o); ssd += __shfl_xor_sync(kFull, ssd, o); }
-    if(lane == 0) { s_sd[c][wid] = sd; s_ssd[c][wid] = ssd; }
-    off += a.rows[c];
+    sd[c] = (int64_t)__ldcg(reinterpret_cast<const unsigned long long*>(&o->sd[c])) * a.mult[c];
+    o->sd[c]  = sd[c];
+    o->ssd[c] = (uint64_t)__ldcg(reinterpret_cast<const unsigned long long*>(&o->ssd[c])) * (uint64_t)a.mult[c];
   }
-  __syncthreads();
-  if(threadIdx.x == 0)
+  #pragma unroll
+  for(int c = 0; c < 4; c++)
   {
-    PairOut* o = a.out;
-    const int nw = blockDim.x >> 5;
-    for(int c = 0; c < 3; c++)
-    {
-      int64_t sd = 0; uint64_t ssd = 0;
-      for(int w = 0; w < nw; w++) { sd += s_sd[c][w]; ssd += s_ssd[c][w]; }
-      o->sd[c]  = sd * a.mult[c];
-      o->ssd[c] = ssd * (uint64_t)a.mult[c];
-    }
-    const double area = (double)a.area;
-    for(int c = 0; c < 4; c++)
-    {
-      int32_t g = 0;
-      if(a.gcd_override_on) { g = a.gcd_override[c]; }
-      else if(a.need_gcd)
-      {
-        const double avg = ddiv(c < 3 ? (double)o->sd[c] : 0.0, area);
-        g = clampi(round_half_away(avg), -a.maxdiff[c], a.maxdiff[c]);
-      }
-      o->gcd[c] = g;
-    }
-    const int inv0 = o->max_sample[0] > (uint32_t)a.maxv;
-    const int inv1 = o->max_sample[1] > (uint32_t)a.maxv;
-    const int int_path = !a.fp32_ok || ((inv0 || inv1) && !a.clip_on);
-    o->flags = inv0 | (inv1 << 1) | (int_path << 2);
+    int32_t g = 0;
+    if(a.gcd_override_on) { g = a.gcd_override[c]; }
+    else if(a.need_gcd) { g = clampi(round_half_away(ddiv((double)sd[c], area)), -a.maxdiff[c], a.maxdiff[c]); }
+    o->gcd[c] = g;
   }
-}
-
-__global__ void __launch_bounds__(1024) k_reduce(const __grid_constant__ ReduceArgs a) { reduce_body(a); }
-
-// one job (frame pair) per CTA
-__global__ void __launch_bounds__(1024) k_reduce_multi(const ReduceArgs* __restrict__ jobs) { reduce_body(jobs[blockIdx.x]); }
-
-cudaError_t launch_reduce(const ReduceArgs& a, cudaStream_t s)
-{
-  k_reduce<<<1, 1024, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_reduce_multi(const ReduceArgs* d_jobs, int njobs, cudaStream_t s)
-{
-  if(njobs <= 0) { return cudaSuccess; }
-  k_reduce_multi<<<njobs, 1024, 0, s>>>(d_jobs);
-  return cudaGetLastError();
+  const int inv0 = __ldcg(&o->max_sample[0]) > (uint32_t)a.maxv;
+  const int inv1 = __ldcg(&o->max_sample[1]) > (uint32_t)a.maxv;
+  const int int_path = !a.fp32_ok || ((inv0 || inv1) && !a.clip_on);
+  o->flags = inv0 | (inv1 << 1) | (int_path << 2);
 }
 
 // (CPS search: qmiv_cps.cu)

@@ -5,7 +5,8 @@
 namespace qmiv {
 
 // ---------------------------------------------------------------------------------------------
-// prepass: per raw row of every plane, SD (In1 - In0) and SSD, plus the largest sample per frame
+// prepass: per raw row of every plane SSD, over the planes SD (In1 - In0), SSD and the largest sample
+// per frame; the last CTA forms the totals, the GCD and the path flags
 // ---------------------------------------------------------------------------------------------
 struct PrepassArgs
 {
@@ -13,29 +14,17 @@ struct PrepassArgs
   int32_t   rows[3];       // raw rows per plane
   int32_t   cols[3];       // raw samples per row per plane
   uint32_t  clip;          // conceal: samples above are clipped (65535 = no clipping)
-  int64_t*  row_sd;        // [rows[0] + rows[1] + rows[2]]
-  uint64_t* row_ssd;       // same indexing
-  PairOut*  out;           // max_sample (atomicMax)
-};
-
-// ---------------------------------------------------------------------------------------------
-// reduce: totals, GCD, path flags
-// ---------------------------------------------------------------------------------------------
-struct ReduceArgs
-{
-  int32_t         rows[3];
-  int32_t         mult[3];     // 4:4:4 multiplicity of a raw chroma sample (1 << (sx + sy))
-  int64_t         area;
-  int32_t         maxv;
-  int32_t         maxdiff[4];  // round(unc * Max) per component, computed on the host in float
-  int32_t         need_gcd;
-  int32_t         gcd_override_on;  // use gcd_override instead of the computed GCD
-  int32_t         gcd_override[4];
-  int32_t         fp32_ok;     // fp32 exact-key CPS path is valid for in-range samples
-  int32_t         clip_on;     // conceal active
-  const int64_t*  row_sd;
-  const uint64_t* row_ssd;
-  PairOut*        out;
+  uint64_t* row_ssd;       // [rows[0] + rows[1] + rows[2]]
+  PairOut*  out;           // zeroed
+  int32_t   mult[3];       // 4:4:4 multiplicity of a raw chroma sample (1 << (sx + sy))
+  int64_t   area;
+  int32_t   maxv;
+  int32_t   maxdiff[4];    // round(unc * Max) per component, computed on the host in float
+  int32_t   need_gcd;
+  int32_t   gcd_override_on;  // use gcd_override instead of the computed GCD
+  int32_t   gcd_override[4];
+  int32_t   fp32_ok;       // the exact-key CPS path is valid for in-range samples
+  int32_t   clip_on;       // conceal active
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -231,7 +220,6 @@ constexpr size_t kFinalizeMaxSmem = 200 * 1024;
 
 // launch wrappers (return cudaError_t of the launch)
 template <typename T> cudaError_t launch_prepass(const PrepassArgs& a, cudaStream_t s);
-cudaError_t launch_reduce(const ReduceArgs& a, cudaStream_t s);
 template <typename T> cudaError_t launch_cps(const CpsArgs& a, int R, cudaStream_t s);
 // Block SSIM launches of one pair (jobs by value) or of many (job tables in device memory, one after the
 // other: pool, img0, imgn, pyr, rows with n entries each)
@@ -260,7 +248,6 @@ size_t      finalize_smem(const FinalizeArgs& a);
 
 // multi-pair forms: argument blocks in device memory, one launch for every pair of a batch
 template <typename T> cudaError_t launch_prepass_multi(const PrepassArgs* d_jobs, int njobs, int max_rows, cudaStream_t s);
-cudaError_t launch_reduce_multi(const ReduceArgs* d_jobs, int njobs, cudaStream_t s);
 size_t      pool_win_elems(int nx, int ny);   // doubles of the windows of nx x ny
 // 16-byte alignment of the moment rows and the scratch, which the pooling kernels copy with cp.async
 bool        pool_job_aligned(const SsimPoolJob& J);

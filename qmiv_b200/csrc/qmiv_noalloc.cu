@@ -26,10 +26,9 @@ constexpr int32_t kMaxH = QMIV_STATIC_MAX_HEIGHT;
 constexpr size_t  kAlign = 256;
 constexpr size_t align_up(size_t n) { return (n + kAlign - 1) & ~(kAlign - 1); }
 
-// scratch layout (bytes): per-row SD / SSD of up to three planes of kMaxH rows, the 32-bit CPS row
+// scratch layout (bytes): per-row SSD of up to three planes of kMaxH rows, the 32-bit CPS row
 // sums of both directions, the device result block, and the ERP row weights
-constexpr size_t kOffRowSd  = 0;
-constexpr size_t kOffRowSsd = kOffRowSd + align_up(sizeof(int64_t) * 3 * kMaxH);
+constexpr size_t kOffRowSsd = 0;
 constexpr size_t kOffCps    = kOffRowSsd + align_up(sizeof(uint64_t) * 3 * kMaxH);
 constexpr size_t kOffOut    = kOffCps + align_up(sizeof(uint32_t) * 2 * 3 * kMaxH);
 constexpr size_t kOffWs     = kOffOut + align_up(sizeof(PairOut));
@@ -51,7 +50,6 @@ template <typename T>
 qmiv_status enqueue_static(char* base, const Shape& S, const qmiv_params& prm, const Img& in0, const Img& in1,
                            uint32_t mask, int32_t ws_rows, cudaStream_t s)
 {
-  int64_t*  row_sd  = reinterpret_cast<int64_t*>(base + kOffRowSd);
   uint64_t* row_ssd = reinterpret_cast<uint64_t*>(base + kOffRowSsd);
   uint32_t* cps     = reinterpret_cast<uint32_t*>(base + kOffCps);
   PairOut*  dout    = reinterpret_cast<PairOut*>(base + kOffOut);
@@ -66,19 +64,15 @@ qmiv_status enqueue_static(char* base, const Shape& S, const qmiv_params& prm, c
   PrepassArgs pa{};
   pa.in0 = in0; pa.in1 = in1;
   for(int c = 0; c < 3; c++) { pa.rows[c] = (int32_t)S.plane_rows(c); pa.cols[c] = (int32_t)S.plane_cols(c); }
-  pa.clip = clip; pa.row_sd = row_sd; pa.row_ssd = row_ssd; pa.out = dout;
-  QMIV_CUDA(launch_prepass<T>(pa, s));
-
+  pa.clip = clip; pa.row_ssd = row_ssd; pa.out = dout;
   int32_t maxdiff[4];
   for(int c = 0; c < 4; c++) { maxdiff[c] = round_f32_half_away(prm.unc[c] * (float)S.maxv); }
-  ReduceArgs ra{};
-  for(int c = 0; c < 3; c++) { ra.rows[c] = pa.rows[c]; ra.mult[c] = c ? (1 << (S.sx + S.sy)) : 1; }
-  ra.area = (int64_t)S.W * S.H; ra.maxv = S.maxv;
-  for(int c = 0; c < 4; c++) { ra.maxdiff[c] = maxdiff[c]; }
-  ra.need_gcd = search; ra.fp32_ok = cps_key_exact(prm.search_range, S.sx, S.sy, S.maxv, prm.cws, maxdiff);
-  ra.clip_on = prm.invalid_pel_action == QMIV_PEL_CNCL;
-  ra.row_sd = row_sd; ra.row_ssd = row_ssd; ra.out = dout;
-  QMIV_CUDA(launch_reduce(ra, s));
+  for(int c = 0; c < 3; c++) { pa.mult[c] = c ? (1 << (S.sx + S.sy)) : 1; }
+  pa.area = (int64_t)S.W * S.H; pa.maxv = S.maxv;
+  for(int c = 0; c < 4; c++) { pa.maxdiff[c] = maxdiff[c]; }
+  pa.need_gcd = search; pa.fp32_ok = cps_key_exact(prm.search_range, S.sx, S.sy, S.maxv, prm.cws, maxdiff);
+  pa.clip_on = prm.invalid_pel_action == QMIV_PEL_CNCL;
+  QMIV_CUDA(launch_prepass<T>(pa, s));
 
   if(search)
   {
