@@ -592,6 +592,7 @@ __device__ __forceinline__ void cps_loop(int ntiles, const Locate& locate, uint3
   __shared__ int16_t s_off[256];
   static_assert(sizeof(CpsArgs) % 4 == 0 && sizeof(CpsGeomArgs) % 4 == 0, "word copies");
 
+  next_may_start();
   if(threadIdx.x == 0) { mbar_init(bar, 1); fence_barrier_init(); }
   build_offsets<R, WY>(s_off);
   __syncthreads();

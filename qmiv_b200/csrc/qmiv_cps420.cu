@@ -690,6 +690,7 @@ __global__ void __launch_bounds__(256, Geo420<R, T, TM>::CTAS) k_cps420(const __
 
   const int warp = __shfl_sync(kFull, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int dir = warp >> 2, by = warp & 3;   // direction and block row of the thread's 4x4 block (column block: lane)
+  next_may_start();
   if(threadIdx.x == 0) { mbar_init(bar, 1); mbar_init(bar + 1, 1); fence_barrier_init(); }
   build_offsets420<R, T>(s_off);
   __syncthreads();

@@ -176,6 +176,14 @@ struct PairOut
   double   ssim[kMaxSsimSlots][3];
 };
 
+// ---- dependent launches ------------------------------------------------------------------------
+// A kernel launched by launch_next may be scheduled while its predecessor in the stream still runs, from
+// when every CTA of that one has called next_may_start. It begins with wait_for_previous, which returns
+// when the predecessor, and so all work before it, is complete and its writes are visible. In an ordinary
+// launch both do nothing.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarriers and bulk copies ----------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

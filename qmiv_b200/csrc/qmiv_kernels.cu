@@ -324,6 +324,7 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a, int chain, 
 __global__ void __launch_bounds__(256) k_finalize(const __grid_constant__ FinalizeArgs a)
 {
   extern __shared__ double stage[];  // [len] values, then [len] ERP weights for weighted SSIM chains
+  wait_for_previous();
   finalize_body(a, blockIdx.x, stage);
 }
 
@@ -331,6 +332,7 @@ __global__ void __launch_bounds__(256) k_finalize(const __grid_constant__ Finali
 __global__ void __launch_bounds__(256) k_finalize_multi(const FinalizeArgs* __restrict__ pairs, const FinJob* __restrict__ jobs)
 {
   extern __shared__ double stage[];
+  wait_for_previous();
   const FinJob j = jobs[blockIdx.x];
   finalize_body(pairs[j.pair], j.chain, stage);
 }
@@ -375,8 +377,7 @@ cudaError_t launch_finalize(const FinalizeArgs& a_in, cudaStream_t s)
   if(smem > kFinalizeMaxSmem) { return cudaErrorInvalidValue; }
   cudaError_t e = finalize_configure();
   if(e != cudaSuccess) { return e; }
-  k_finalize<<<blocks, 256, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_next(k_finalize, blocks, 256, smem, s, a);
 }
 
 cudaError_t launch_finalize_multi(const FinalizeArgs* d_pairs, const FinJob* d_jobs, int njobs, size_t smem, cudaStream_t s)
@@ -385,8 +386,7 @@ cudaError_t launch_finalize_multi(const FinalizeArgs* d_pairs, const FinJob* d_j
   if(smem > kFinalizeMaxSmem) { return cudaErrorInvalidValue; }
   cudaError_t e = finalize_configure();
   if(e != cudaSuccess) { return e; }
-  k_finalize_multi<<<njobs, 256, smem, s>>>(d_pairs, d_jobs);
-  return cudaGetLastError();
+  return launch_next(k_finalize_multi, njobs, 256, smem, s, d_pairs, d_jobs);
 }
 
 }  // namespace qmiv

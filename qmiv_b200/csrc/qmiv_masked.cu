@@ -986,15 +986,15 @@ __device__ __forceinline__ void mask_finalize_body(const MaskArgs& a, int chain)
 // ---- kernels: one frame pair (arguments in parameter space) and many (a device table of arguments,
 // one grid dimension indexing the pair; CTAs beyond their pair's extent return) -----------------
 template <typename T, typename TM>
-__global__ void __launch_bounds__(256) k_mask_prepass(const __grid_constant__ MaskArgs a) { mask_prepass_body<T, TM>(a, blockIdx.x); }
+__global__ void __launch_bounds__(256) k_mask_prepass(const __grid_constant__ MaskArgs a) { next_may_start(); mask_prepass_body<T, TM>(a, blockIdx.x); }
 template <typename T, typename TM>
-__global__ void __launch_bounds__(256, 2) k_mask_prepass420v(const __grid_constant__ MaskArgs a) { mask_prepass420_body<T, TM>(a, blockIdx.x); }
-__global__ void k_mask_reduce(const __grid_constant__ MaskArgs a) { mask_reduce_body(a); }
+__global__ void __launch_bounds__(256, 2) k_mask_prepass420v(const __grid_constant__ MaskArgs a) { next_may_start(); mask_prepass420_body<T, TM>(a, blockIdx.x); }
+__global__ void k_mask_reduce(const __grid_constant__ MaskArgs a) { wait_for_previous(); mask_reduce_body(a); }
 template <typename T, typename TM, int R>
 __global__ void __launch_bounds__(256) k_cps_masked(const __grid_constant__ MaskArgs a) { cps_masked_body<T, TM, R>(a, blockIdx.x, blockIdx.y, blockIdx.z); }
 template <typename T, typename TM, int R>
 __global__ void __launch_bounds__(512, 2) k_cps_masked_key(const __grid_constant__ MaskArgs a) { cps_masked_key_body<T, TM, R>(a, blockIdx.x, blockIdx.y, a.kscale); }
-__global__ void __launch_bounds__(256) k_mask_finalize(const __grid_constant__ MaskArgs a) { mask_finalize_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(256) k_mask_finalize(const __grid_constant__ MaskArgs a) { wait_for_previous(); mask_finalize_body(a, blockIdx.x); }
 
 // The arguments of up to kPackPairs pairs of one launch group, passed by value: every CTA reads its
 // pair's arguments from the constant bank as the one-pair kernels do, without a dependent global load.
@@ -1009,11 +1009,12 @@ static_assert(sizeof(MaskPack) <= 32000, "kernel parameters are limited to 32 KB
 template <typename T, typename TM, bool VEC>
 __global__ void __launch_bounds__(256, 2) k_mask_prepass_multi(const __grid_constant__ MaskPack pk)
 {
+  next_may_start();
   const MaskArgs& a = pk.a[blockIdx.y];
   if((int)blockIdx.x >= (VEC ? prepass420_units<TM>(a.H) : a.H)) { return; }
   if(VEC) { mask_prepass420_body<T, TM>(a, blockIdx.x); } else { mask_prepass_body<T, TM>(a, blockIdx.x); }
 }
-__global__ void k_mask_reduce_multi(const __grid_constant__ MaskPack pk) { mask_reduce_body(pk.a[blockIdx.x]); }
+__global__ void k_mask_reduce_multi(const __grid_constant__ MaskPack pk) { wait_for_previous(); mask_reduce_body(pk.a[blockIdx.x]); }
 template <typename T, typename TM, int R>
 __global__ void __launch_bounds__(256) k_cps_masked_multi(const __grid_constant__ MaskPack pk)
 {
@@ -1030,6 +1031,7 @@ __global__ void __launch_bounds__(512, 2) k_cps_masked_key_multi(const __grid_co
 }
 __global__ void __launch_bounds__(256) k_mask_finalize_multi(const __grid_constant__ MaskPack pk)
 {
+  wait_for_previous();
   mask_finalize_body(pk.a[blockIdx.x / 9], blockIdx.x % 9);
 }
 
@@ -1070,7 +1072,7 @@ cudaError_t launch_masked_t(const MaskArgs& a, int R, bool key, const CpsArgs* c
   else { k_mask_prepass<T, TM><<<a.H, 256, 0, s>>>(a); }
   pipe.prof_end(s, QMIV_STAGE_PREPASS, tok);
   tok = pipe.prof_begin(s);
-  k_mask_reduce<<<1, 32, 0, s>>>(a);
+  { const cudaError_t e = launch_next(k_mask_reduce, 1, 32, 0, s, a); if(e != cudaSuccess) { return e; } }
   pipe.prof_end(s, QMIV_STAGE_REDUCE, tok);
   tok = pipe.prof_begin(s);
   const dim3 grid((a.W + 31) / 32, (a.H + 7) / 8, 2);
@@ -1104,7 +1106,7 @@ cudaError_t launch_masked_t(const MaskArgs& a, int R, bool key, const CpsArgs* c
   }
   pipe.prof_end(s, QMIV_STAGE_CPS, tok);
   tok = pipe.prof_begin(s);
-  k_mask_finalize<<<9, 256, 0, s>>>(a);
+  { const cudaError_t e = launch_next(k_mask_finalize, 9, 256, 0, s, a); if(e != cudaSuccess) { return e; } }
   pipe.prof_end(s, QMIV_STAGE_FINALIZE, tok);
   return cudaGetLastError();
 }
@@ -1543,7 +1545,7 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
   }
   clock_.end(s, QMIV_STAGE_PREPASS, tok);
   tok = clock_.begin(ctx, s);
-  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); k_mask_reduce_multi<<<cnt, 32, 0, s>>>(pk); }
+  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); QMIV_CUDA(launch_next(k_mask_reduce_multi, cnt, 32, 0, s, pk)); }
   clock_.end(s, QMIV_STAGE_REDUCE, tok);
   tok = clock_.begin(ctx, s);
   for(auto& g : srch)
@@ -1568,7 +1570,7 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
   }
   clock_.end(s, QMIV_STAGE_CPS, tok);
   tok = clock_.begin(ctx, s);
-  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); k_mask_finalize_multi<<<9 * cnt, 256, 0, s>>>(pk); }
+  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); QMIV_CUDA(launch_next(k_mask_finalize_multi, 9 * cnt, 256, 0, s, pk)); }
   clock_.end(s, QMIV_STAGE_FINALIZE, tok);
   QMIV_CUDA(cudaGetLastError());
   tok = clock_.begin(ctx, s);
