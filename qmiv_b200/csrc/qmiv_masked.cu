@@ -917,15 +917,15 @@ __device__ __forceinline__ void cps_masked_key_body(const MaskArgs& a, int bx, i
 }
 
 // Chains 0..2: WS rows of component c; chains 3..8: CPS rows of (direction, component). Each is the
-// reference's row-order compensated sum; the CPS chains also form the plain uint64 totals. One CTA per
-// chain: all threads stage a chunk of the chain's terms (the products with the ERP weights, the same
-// doubles the serial loop would form) in shared memory, then thread 0 adds them in row order, so the
-// serial chain never waits on global memory.
+// reference's row-order compensated sum, formed by all threads of its CTA (ExactSum); the CPS chains
+// also form the plain uint64 totals. A chain whose order matters is staged in shared memory chunk by chunk and
+// added by one thread. 4096x2048: 22 us by one thread per chain, 8.6 like this.
 constexpr int kMaskFinChunk = 4096;
 __device__ __forceinline__ void mask_finalize_body(const MaskArgs& a, int chain)
 {
   __shared__ double vals[kMaskFinChunk];
-  __shared__ unsigned long long tot, top;
+  __shared__ unsigned long long tot;
+  __shared__ ExactSum part[8];
   const int k = chain;
   if(k < 3 && !a.ws) { return; }                              // uniform over the CTA
   MaskOut* o = a.out;
@@ -936,40 +936,44 @@ __device__ __forceinline__ void mask_finalize_body(const MaskArgs& a, int chain)
   const size_t step = cps ? 3 : 1;
   if(threadIdx.x == 0) { tot = 0ull; }
   unsigned long long loc = 0ull;
-  Kbns s;                                                     // used by thread 0
+  ExactSum es;
   for(int base = 0; base < H; base += kMaskFinChunk)
   {
-    const int n = min(kMaskFinChunk, H - base);
-    __syncthreads();                                          // the previous chunk has been summed
-    if(threadIdx.x == 0) { top = 0ull; }
-    __syncthreads();
-    unsigned long long tv = 0ull;
     constexpr int U = kMaskFinChunk / 256;                    // a thread's loads all in flight at once
     uint64_t v[U];
     double w[U];
     #pragma unroll
     for(int u = 0; u < U; u++)
     {
-      const int i = threadIdx.x + u * 256;
-      v[u] = i < n ? r[(size_t)(base + i) * step] : 0ull;
-      w[u] = (i < n && a.ws) ? a.ws[base + i] : 0.0;
+      const int i = base + threadIdx.x + u * 256;
+      v[u] = i < H ? r[(size_t)i * step] : 0ull;
+      w[u] = (i < H && a.ws) ? a.ws[i] : 0.0;
     }
     #pragma unroll
     for(int u = 0; u < U; u++)
     {
-      const int i = threadIdx.x + u * 256;
-      if(i < n)
-      {
-        loc += v[u];
-        vals[i] = a.ws ? dmul((double)v[u], w[u]) : 0.0;
-        tv = max(tv, term_bits(vals[i]));
-      }
+      loc += v[u];
+      if(a.ws) { es.add(dmul((double)v[u], w[u])); }
     }
-    #pragma unroll
-    for(int o2 = 16; o2 > 0; o2 >>= 1) { tv = max(tv, __shfl_xor_sync(0xffffffffu, tv, o2)); }
-    if((threadIdx.x & 31) == 0) { atomicMax(&top, tv); }
-    __syncthreads();
-    if(threadIdx.x == 0 && a.ws) { chain_sum(s, vals, n, top); }
+  }
+  es.join_warp();
+  if((threadIdx.x & 31) == 0) { part[threadIdx.x >> 5] = es; }
+  __syncthreads();
+  es = part[0];
+  for(int q = 1; q < 8; q++) { es.join(part[q]); }            // the same for every thread
+  double total = es.result();
+  if(!es.exact(H))                                            // uniform: the chain in order, by thread 0
+  {
+    Kbns s;
+    for(int base = 0; base < H; base += kMaskFinChunk)
+    {
+      const int n = min(kMaskFinChunk, H - base);
+      __syncthreads();                                        // the previous chunk has been summed
+      for(int i = threadIdx.x; i < n; i += 256) { vals[i] = dmul((double)r[(size_t)(base + i) * step], a.ws[base + i]); }
+      __syncthreads();
+      if(threadIdx.x == 0) { chain_sum(s, vals, n, es); }
+    }
+    total = s.result();
   }
   loc = warp_sum_u64(loc);                                    // exact: integer sum in any order
   if((threadIdx.x & 31) == 0) { atomicAdd(&tot, loc); }
@@ -978,9 +982,9 @@ __device__ __forceinline__ void mask_finalize_body(const MaskArgs& a, int chain)
   if(cps)
   {
     o->cps_sum[d][c] = tot;
-    o->cps_ws[d][c] = a.ws ? s.result() : 0.0;
+    o->cps_ws[d][c] = total;
   }
-  else { o->ws_err[k] = s.result(); }
+  else { o->ws_err[k] = total; }
 }
 
 // ---- kernels: one frame pair (arguments in parameter space) and many (a device table of arguments,

@@ -6,8 +6,8 @@
 // pictures themselves, evaluates the windows there and writes the next scale's 2x2 means
 // (xPixelOpsSTD.cpp:50-67) on the way: no moment planes in device memory. k_ssim_pyr makes the scales
 // below from the first of them, so that one launch takes the windows of all smaller scales. Windows are
-// evaluated in FP64 with the reference's operation order; k_ssim_rows sums each window row in x order with
-// the compensated sum, one lane per row, all scales and pairs in one launch.
+// evaluated in FP64 with the reference's operation order; k_ssim_rows forms the compensated sum of each
+// window row, all scales and pairs in one launch.
 // Measured against moment planes in device memory and three launches per scale: 8 pairs of 2048x2048 10-bit,
 // MS-SSIM and IV-MS-SSIM, 827 -> 523 us of device time; one 1998x1080 12-bit pair, every metric, 33 -> 9
 // launches and 262 -> 98 us. What bounds k_ssim_img: load latency and issue (58 % at 32 warps per SM; 4 CTAs
@@ -19,7 +19,7 @@
 namespace qmiv {
 
 // =============================================================================================
-// windows + ordered row sums (xSSIM.cpp:353-369), two kernels:
+// windows + row sums (xSSIM.cpp:353-369), two kernels:
 //   k_ssim_win   a CTA (eight warps) evaluates the windows [x0, x0 + 64) of one band of 32 window rows.
 //                The 33 block rows x 68 columns of the five moment planes it needs (45 KB) are staged
 //                in shared memory by cp.async, all in flight at once. Lane l then takes columns
@@ -28,10 +28,7 @@ namespace qmiv {
 //                Each window is evaluated in FP64 with the reference's operation order; the 64 x 32
 //                values reuse the staging space and leave as 16 contiguous KB of the job's scratch
 //                [band][x][32].
-//   k_ssim_rows  one warp per band, lane j summing window row 32 band + j in x order with the
-//                compensated sum. 8 KB chunks of 32 columns are staged in shared memory by cp.async,
-//                three in flight per warp, so the serial chain never waits for DRAM.
-// All windows are independent work for the first kernel; only the second is order-dependent.
+//   k_ssim_rows  a CTA per band of 32 window rows forms their sums (ExactSum).
 // =============================================================================================
 constexpr int kWinX = 64;                                  // windows per CTA in x
 constexpr int kWinNT = 256;                                // threads per CTA
@@ -40,8 +37,7 @@ constexpr int kWinOcc = 5, kImgOcc = 4;                    // CTAs per SM of k_s
 constexpr int kStRows = 33;                                // block rows of a band
 constexpr int kStCols = 68;                                // block columns staged (65 used), 16-byte pieces
 constexpr int kStPieces = kStCols / 4;
-constexpr int kRowCols = 32;                               // columns per staged chunk of k_ssim_rows
-constexpr int kRowStages = 4;
+constexpr int kRowWarps = 8;                               // of k_ssim_rows
 static_assert(kWinX * 33 * sizeof(double) <= 5 * kStRows * kStCols * sizeof(uint32_t), "values fit the staging space");
 
 size_t pool_win_elems(int nx, int ny) { return (size_t)((ny + 31) / 32) * 32 * (size_t)nx; }
@@ -446,59 +442,53 @@ __device__ __forceinline__ void ssim_pyr_any(const SsimPyrJob& J, int bx, int by
   else { ssim_pyr_body<uint16_t>(J, l2, l3, bx, by); }
 }
 
+// Sums of the window values along the rows: a CTA per band of 32 rows, a lane per row, the columns dealt to
+// the warps. A column of a band is 256 contiguous bytes. Bound by the latency of the loads with few bands and
+// by reading the values from memory with many: with one warp per band, summing in order behind copies
+// into shared memory, 25 us for the six evaluations of a 4096x2048 pair and 40 for eight pairs (200 MB); now
+// 12.6 and 42.6. With 16 warps 12.7 and 45.4, with 4 21 and 43, with eight loads in flight 14.7 and 49.9.
 __device__ __forceinline__ void ssim_rows_body(const SsimRowJob& J, int band)
 {
-  __shared__ __align__(16) double st[kRowStages][kRowCols][32];   // [stage][column][row in band]
-  const int lane = threadIdx.x & 31;
-  if(band * 32 >= J.ny) { return; }                         // one warp per CTA: uniform
-  const char* src = reinterpret_cast<const char*>(J.win + (size_t)band * J.nx * 32);
-  const int nchunks = (J.nx + kRowCols - 1) / kRowCols;
-  // chunk c: columns [32 c, min(32 c + 32, nx)), 256 bytes each, contiguous in the scratch
-  auto issue = [&](int c) {
-    if(c < nchunks)
-    {
-      const int pieces = min(kRowCols, J.nx - c * kRowCols) * 16;
-      char* dst = reinterpret_cast<char*>(st[c % kRowStages]);
-      const char* s = src + (size_t)c * kRowCols * 256;
-      for(int q = lane; q < pieces; q += 32) { cp_async16(dst + 16 * q, s + 16 * q); }
-    }
-    cp_async_commit();                                      // empty groups keep the count uniform
-  };
-  #pragma unroll
-  for(int c = 0; c < kRowStages - 1; c++) { issue(c); }
-  Kbns row;
-  for(int c = 0; c < nchunks; c++)
+  __shared__ ExactSum part[kRowWarps / 2][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if(band * 32 >= J.ny) { return; }                         // uniform over the CTA
+  const double* src = J.win + (size_t)band * J.nx * 32 + lane;
+  constexpr int U = 16;                                     // loads in flight per thread
+  ExactSum sum;
+  for(int x0 = warp; x0 < J.nx; x0 += U * kRowWarps)
   {
-    cp_async_wait<kRowStages - 2>();                        // chunk c has landed (this lane's part)
-    __syncwarp();                                           // ... and every other lane's
-    const int cols = min(kRowCols, J.nx - c * kRowCols);
-    const double (*b)[32] = st[c % kRowStages];
-    // Window values lie within [-2, 2] (|cov| <= (var_r + var_t) / 2 up to rounding far below C2), so a sum of
-    // at least 2 (kRowCols + 1) stays above every term of the chunk; rows past the last one hold zeros or
-    // nothing and are not written
-    if(cols == kRowCols && __all_sync(0xffffffffu, band * 32 + lane >= J.ny || row.s >= 2.0 * (kRowCols + 1)))
-    {
-      double v[kRowCols];
-      #pragma unroll
-      for(int x = 0; x < kRowCols; x++) { v[x] = b[x][lane]; }
-      row.add_small(v);
-    }
-    else if(cols == kRowCols)
-    {
-      // straight-line code: the loads and the non-carried parts of the sums overlap the chain
-      #pragma unroll
-      for(int x = 0; x < kRowCols; x++) { row.add(b[x][lane]); }
-    }
-    else
-    {
-      #pragma unroll 1
-      for(int x = 0; x < cols; x++) { row.add(b[x][lane]); }
-    }
-    __syncwarp();                                           // every lane is past its reads of chunk c - 1
-    issue(c + kRowStages - 1);                              // into the stage that chunk c - 1 used
+    double v[U];
+    #pragma unroll
+    for(int u = 0; u < U; u++) { const int x = x0 + u * kRowWarps; v[u] = x < J.nx ? src[(size_t)x * 32] : 0.0; }
+    #pragma unroll
+    for(int u = 0; u < U; u++) { sum.add(v[u]); }
   }
+  #pragma unroll
+  for(int half = kRowWarps / 2; half > 0; half >>= 1)        // warps in [half, 2 half) hand theirs over
+  {
+    if(warp >= half) { if(warp < 2 * half) { part[warp - half][lane] = sum; } }
+    __syncthreads();
+    if(warp < half) { sum.join(part[warp][lane]); }
+    if(half > 1) { __syncthreads(); }
+  }
+  if(warp != 0) { return; }
   const int j = band * 32 + lane;
-  if(j < J.ny) { J.row_sum[j] = row.result(); }
+  const bool valid = j < J.ny;                              // rows past the last one hold zeros or nothing
+  double r = sum.result();
+  if(__any_sync(0xffffffffu, valid && !sum.exact(J.nx)))
+  {
+    Kbns row;                                               // the chain in order, loads ahead of it
+    for(int x0 = 0; x0 < J.nx; x0 += 16)
+    {
+      double v[16];
+      #pragma unroll
+      for(int u = 0; u < 16; u++) { v[u] = x0 + u < J.nx ? src[(size_t)(x0 + u) * 32] : 0.0; }
+      #pragma unroll
+      for(int u = 0; u < 16; u++) { if(x0 + u < J.nx) { row.add(v[u]); } }
+    }
+    r = row.result();
+  }
+  if(valid) { J.row_sum[j] = r; }
 }
 
 // Every kernel takes its jobs by value (one pair) or from a table in device memory. The job is the fastest
@@ -516,8 +506,8 @@ __global__ void __launch_bounds__(kWinNT, kImgOcc) k_ssim_img(const __grid_const
 __global__ void __launch_bounds__(kWinNT, kImgOcc) k_ssim_img_multi(const SsimImgJob* __restrict__ jobs) { ssim_img_any(jobs[blockIdx.x], blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(256) k_ssim_pyr(const __grid_constant__ JobArgs<SsimPyrJob, kMaxPyrJobs> a) { ssim_pyr_any(a.job[blockIdx.z], blockIdx.x, blockIdx.y); }
 __global__ void __launch_bounds__(256) k_ssim_pyr_multi(const SsimPyrJob* __restrict__ jobs) { ssim_pyr_any(jobs[blockIdx.z], blockIdx.x, blockIdx.y); }
-__global__ void __launch_bounds__(32) k_ssim_rows(const __grid_constant__ JobArgs<SsimRowJob, kMaxRowJobs> a) { next_may_start(); ssim_rows_body(a.job[blockIdx.y], blockIdx.x); }
-__global__ void __launch_bounds__(32) k_ssim_rows_multi(const SsimRowJob* __restrict__ jobs) { next_may_start(); ssim_rows_body(jobs[blockIdx.y], blockIdx.x); }
+__global__ void __launch_bounds__(32 * kRowWarps, 3) k_ssim_rows(const __grid_constant__ JobArgs<SsimRowJob, kMaxRowJobs> a) { next_may_start(); ssim_rows_body(a.job[blockIdx.y], blockIdx.x); }
+__global__ void __launch_bounds__(32 * kRowWarps, 3) k_ssim_rows_multi(const SsimRowJob* __restrict__ jobs) { next_may_start(); ssim_rows_body(jobs[blockIdx.y], blockIdx.x); }
 
 // ---- host ---------------------------------------------------------------------------------------
 static int tiles_of(int nx) { return (nx + kWinX - 1) / kWinX; }
@@ -649,12 +639,8 @@ cudaError_t launch_ssim_rows(const JobArgs<SsimRowJob, kMaxRowJobs>& a, int njob
 {
   if(njobs <= 0) { return cudaSuccess; }
   int maxny = 0;
-  for(int k = 0; k < njobs; k++)
-  {
-    if(((uintptr_t)a.job[k].win & 15) != 0) { return cudaErrorMisalignedAddress; }
-    maxny = max(maxny, a.job[k].ny);
-  }
-  k_ssim_rows<<<dim3(bands_of(maxny), njobs), 32, 0, s>>>(a);
+  for(int k = 0; k < njobs; k++) { maxny = max(maxny, a.job[k].ny); }
+  k_ssim_rows<<<dim3(bands_of(maxny), njobs), 32 * kRowWarps, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -678,7 +664,7 @@ cudaError_t launch_ssim_tables(const SsimTables& t, cudaStream_t s, bool rows_on
   cudaError_t e = cudaSuccess;
   if(rows_only)
   {
-    if(t.nrows) { k_ssim_rows_multi<<<dim3(bands_of(d.rows_ny), t.nrows), 32, 0, s>>>(t.rows); e = last_or(e); }
+    if(t.nrows) { k_ssim_rows_multi<<<dim3(bands_of(d.rows_ny), t.nrows), 32 * kRowWarps, 0, s>>>(t.rows); e = last_or(e); }
     return e;
   }
   if(e == cudaSuccess && t.npool) { e = launch_next(k_ssim_win_multi, dim3(tiles_of(d.pool_nx), bands_of(d.pool_ny), t.npool), kWinNT, 0, s, t.pool); }
