@@ -394,8 +394,10 @@ qmiv_status PairPipeline::enqueue_t(const Img& in0, const Img& in1, uint32_t mas
   fa.do_wspsnr = (mask & QMIV_WSPSNR) ? 1 : 0;
   fa.cps_rows = need_search ? rows_device() : nullptr;
   fa.out = dout;
+  const bool chains = finalize_plan(fa) > 0;
+  if(chains) { fa.host = h_out; }                           // pinned: the kernel writes the results there itself
   { const int t = prof_begin(s); QMIV_CUDA(launch_finalize(fa, s)); prof_end(s, QMIV_STAGE_FINALIZE, t); }
-  { const int t = prof_begin(s); QMIV_CUDA(cudaMemcpyAsync(h_out, dout, sizeof(PairOut), cudaMemcpyDeviceToHost, s)); prof_end(s, QMIV_STAGE_D2H, t); }
+  if(!chains) { const int t = prof_begin(s); QMIV_CUDA(cudaMemcpyAsync(h_out, dout, sizeof(PairOut), cudaMemcpyDeviceToHost, s)); prof_end(s, QMIV_STAGE_D2H, t); }
   return QMIV_OK;
 }
 

@@ -289,7 +289,7 @@ public:
   ~MaskedPipeline();
 
 private:
-  DevMem out_, rows_, stage_;
+  DevMem out_, stage_;
   void*  h_out_ = nullptr;
 };
 

@@ -196,6 +196,7 @@ __device__ __forceinline__ void prepass_totals(const PrepassArgs& a)
   const int inv1 = __ldcg(&o->max_sample[1]) > (uint32_t)a.maxv;
   const int int_path = !a.fp32_ok || ((inv0 || inv1) && !a.clip_on);
   o->flags = inv0 | (inv1 << 1) | (int_path << 2);
+  o->done = 0u;
 }
 
 // (CPS search: qmiv_cps.cu)
@@ -333,6 +334,19 @@ __global__ void __launch_bounds__(256) k_finalize(const __grid_constant__ Finali
   extern __shared__ double stage[];  // [len] values, then [len] ERP weights for weighted SSIM chains
   wait_for_previous();
   finalize_body(a, blockIdx.x, stage);
+  if(a.host == nullptr) { return; }
+  // The CTA that finishes last writes the results to the host: a copy behind the kernel took 5 us more.
+  __shared__ bool last;
+  __syncthreads();
+  if(threadIdx.x == 0) { __threadfence(); last = atomicAdd(&a.out->done, 1u) == gridDim.x - 1u; }
+  __syncthreads();
+  if(!last) { return; }
+  __threadfence();
+  static_assert(sizeof(PairOut) % 4 == 0, "word copies");
+  for(int w = threadIdx.x; w < (int)(sizeof(PairOut) / 4); w += blockDim.x)
+  {
+    reinterpret_cast<volatile uint32_t*>(a.host)[w] = __ldcg(reinterpret_cast<const uint32_t*>(a.out) + w);
+  }
 }
 
 // one (pair, chain) job per CTA

@@ -209,6 +209,7 @@ struct FinalizeArgs
   int32_t         nchains;              // filled by launch_finalize
   FinChain        chain[3 + 6 + 3 * kMaxSsimSlots];
   PairOut*        out;
+  PairOut*        host;                 // one pair: pinned host memory the finished results are written to, or null
 };
 
 // The pictures, buffers and sizes of one pair's block SSIM family

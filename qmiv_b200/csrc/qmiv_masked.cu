@@ -1311,15 +1311,16 @@ qmiv_status MaskedPipeline::run(qmiv_calc_s* calc, const qmiv_frame* in0, const 
   Img a0{}, a1{};
   QMIV_TRY(pipe.resolve(in0, 0, a0, s));
   QMIV_TRY(pipe.resolve(in1, 1, a1, s));
-  QMIV_TRY(out_.ensure(calc->ctx, sizeof(MaskOut)));
-  QMIV_TRY(rows_.ensure(calc->ctx, (size_t)9 * S.H * sizeof(uint64_t)));
+  // the result block, then the row sums, cleared by one memset
+  constexpr size_t rows_off = (sizeof(MaskOut) + 255) & ~(size_t)255;
+  const size_t out_bytes = rows_off + (size_t)9 * S.H * sizeof(uint64_t);
+  QMIV_TRY(out_.ensure(calc->ctx, out_bytes));
   if(!h_out_) { QMIV_CUDA(cudaMallocHost(&h_out_, sizeof(MaskOut))); }
   MaskArgs a{};
   if(mask->mem == QMIV_MEM_HOST) { QMIV_TRY(stage_.ensure(calc->ctx, (size_t)S.W * P.mesz * S.H)); }
   QMIV_TRY(resolve_mask(P, mask, stage_.as<char>(), a, s));
-  fill_mask_args(P, a0, a1, rows_.as<uint64_t>(), pipe.ws_device(), out_.as<MaskOut>(), a);
-  QMIV_CUDA(cudaMemsetAsync(out_.p, 0, sizeof(MaskOut), s));
-  QMIV_CUDA(cudaMemsetAsync(a.row_cps, 0, (size_t)6 * S.H * sizeof(uint64_t), s));
+  fill_mask_args(P, a0, a1, reinterpret_cast<uint64_t*>(out_.as<char>() + rows_off), pipe.ws_device(), out_.as<MaskOut>(), a);
+  QMIV_CUDA(cudaMemsetAsync(out_.p, 0, out_bytes, s));
   const int R = P.prm.search_range;
   const CpsArgs ca = mask_cps_args(P, a);
   const CpsArgs* c420 = P.key420 ? &ca : nullptr;
