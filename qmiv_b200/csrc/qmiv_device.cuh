@@ -224,7 +224,7 @@ struct PairOut
   int32_t  gcd[4];
   int32_t  flags;            // bit0: frame0 invalid, bit1: frame1 invalid, bit2: integer CPS path,
                              // bit3: a CPS tile load did not complete (bounded wait ran out)
-  uint32_t max_sample[2];
+  uint32_t or_sample[2];     // OR of every sample per frame: above maxv (2^bd - 1) iff some sample is
   uint32_t done;             // CTAs of the prepass that have added their rows; then chains finished
   int64_t  sd[3];            // 4:4:4 totals of In1 - In0 (raw sums while the prepass runs)
   uint64_t ssd[3];           // 4:4:4 totals

@@ -24,6 +24,37 @@ constexpr unsigned kFull = 0xffffffffu;
 // A warp takes one raw row. Its sums join the picture's by way of the CTA (eight rows, six additions to the
 // result block), and the CTA that adds last turns the totals into the GCD (xGlobClrDiff.cpp:70-103) and the
 // path flags: a launch of its own for that took 7 us of a one-pair call, most of it latency.
+// Bound by the loads' latency for one pair and near the memory's rate for many: with one 16-byte load of each row in
+// flight, 64-bit sums per sample and only rows that start on 16 bytes, 4096x2048 10 bits took 25.6 us (eight
+// pairs, 400 MB, 79); like this 21.4 (71). A 1998x1080 12-bit call, whose rows start anywhere: 227 -> 218 us.
+// Sum and sum of squares of B - A over the samples of one 16-byte vector of either row (8-bit samples: Gram
+// sums by byte dot products; 16-bit samples below 2^14: both differences of a word from one subtraction).
+template <typename T>
+__device__ __forceinline__ void prepass_vector(const uint32_t (&A)[4], const uint32_t (&B)[4], int32_t& d, uint32_t& dd)
+{
+  uint32_t sa = 0, sb = 0, qq = 0, ab = 0;
+  d = 0; dd = 0;
+  #pragma unroll
+  for(int k = 0; k < 4; k++)
+  {
+    if constexpr(sizeof(T) == 1)
+    {
+      sa = __dp4a(A[k], 0x01010101u, sa);
+      sb = __dp4a(B[k], 0x01010101u, sb);
+      qq = __dp4a(A[k], A[k], __dp4a(B[k], B[k], qq));
+      ab = __dp4a(A[k], B[k], ab);
+    }
+    else
+    {
+      const int32_t w = (int32_t)(B[k] - A[k]), lo = (int16_t)w, hi = (w + 0x8000) >> 16;   // |lo| < 2^14 borrows nothing from the rounding
+      d += lo + hi;
+      dd += (uint32_t)(lo * lo);
+      dd += (uint32_t)(hi * hi);                             // eight squares below 2^28
+    }
+  }
+  if constexpr(sizeof(T) == 1) { d = (int32_t)(sb - sa); dd = qq - 2u * ab; }
+}
+
 template <typename T>
 __device__ __forceinline__ void prepass_row(const PrepassArgs& a, int warp, int lane, int& c, int64_t& sd_out, uint64_t& ssd_out, uint32_t& m0_out,
                                             uint32_t& m1_out)
@@ -37,53 +68,81 @@ __device__ __forceinline__ void prepass_row(const PrepassArgs& a, int warp, int 
 
   int64_t  sd  = 0;
   uint64_t ssd = 0;
-  uint32_t m0 = 0, m1 = 0;
+  uint32_t m0 = 0, m1 = 0;                                 // OR of the samples
   auto sample = [&](uint32_t v0, uint32_t v1) {
-    m0 = max(m0, v0); m1 = max(m1, v1);
     v0 = min(v0, a.clip); v1 = min(v1, a.clip);
     const int32_t d = (int32_t)v1 - (int32_t)v0;
     sd  += d;
     ssd += (uint32_t)d * (uint32_t)d;                    // d^2 < 2^32 for 16-bit samples
   };
-  // 16-byte loads where both rows allow them (each lane then holds 8 or 16 samples of each frame in
-  // flight), the rest of the row sample by sample
-  int x0 = 0;
-  if((((uintptr_t)p0 | (uintptr_t)p1) & 15) == 0)
+  // 16-byte loads, four of each row in flight per lane, where both rows lie alike to 16 bytes; what is before the first
+  // boundary and behind the last sample by sample
+  int head = 0, x0 = 0;
+  if((((uintptr_t)p0 ^ (uintptr_t)p1) & 15) == 0)
   {
-    constexpr int V = 16 / (int)sizeof(T);
-    const int nv = n / V;
-    const uint4* q0 = reinterpret_cast<const uint4*>(p0);
-    const uint4* q1 = reinterpret_cast<const uint4*>(p1);
-    for(int v = lane; v < nv; v += 32)
+    constexpr int V = 16 / (int)sizeof(T), U = 4;
+    head = min(n, (int)((0u - (uint32_t)(uintptr_t)p0) & 15u) / (int)sizeof(T));
+    const int nv = (n - head) / V;
+    const uint4* q0 = reinterpret_cast<const uint4*>(p0 + head);
+    const uint4* q1 = reinterpret_cast<const uint4*>(p1 + head);
+    const bool clips = a.clip < (sizeof(T) == 1 ? 0xffu : 0xffffu);
+    for(int v0 = lane; v0 < nv; v0 += 32 * U)
     {
-      const uint4 A = __ldg(q0 + v), B = __ldg(q1 + v);
-      const uint32_t wa[4] = { A.x, A.y, A.z, A.w }, wb[4] = { B.x, B.y, B.z, B.w };
+      uint4 A[U], B[U];
       #pragma unroll
-      for(int k = 0; k < 4; k++)
+      for(int u = 0; u < U; u++)
       {
-        if(sizeof(T) == 2)
+        const int v = v0 + 32 * u;
+        A[u] = B[u] = make_uint4(0u, 0u, 0u, 0u);          // equal samples add nothing
+        if(v < nv) { A[u] = __ldg(q0 + v); B[u] = __ldg(q1 + v); }
+      }
+      #pragma unroll
+      for(int u = 0; u < U; u++)
+      {
+        const uint32_t wa[4] = { A[u].x, A[u].y, A[u].z, A[u].w }, wb[4] = { B[u].x, B[u].y, B[u].z, B[u].w };
+        const uint32_t oa = wa[0] | wa[1] | wa[2] | wa[3], ob = wb[0] | wb[1] | wb[2] | wb[3];
+        m0 |= oa; m1 |= ob;
+        if(!clips && (sizeof(T) == 1 || ((oa | ob) & 0xc000c000u) == 0u))
         {
-          sample(wa[k] & 0xffffu, wb[k] & 0xffffu);
-          sample(wa[k] >> 16, wb[k] >> 16);
+          int32_t d;
+          uint32_t dd;
+          prepass_vector<T>(wa, wb, d, dd);
+          sd += d; ssd += dd;
         }
         else
         {
-          #pragma unroll
-          for(int b = 0; b < 4; b++) { sample((wa[k] >> (8 * b)) & 0xffu, (wb[k] >> (8 * b)) & 0xffu); }
+          #pragma unroll 1
+          for(int k = 0; k < V; k++)
+          {
+            constexpr int BITS = 8 * (int)sizeof(T);
+            const uint32_t w0 = k * BITS < 64 ? (k * BITS < 32 ? wa[0] : wa[1]) : (k * BITS < 96 ? wa[2] : wa[3]);
+            const uint32_t w1 = k * BITS < 64 ? (k * BITS < 32 ? wb[0] : wb[1]) : (k * BITS < 96 ? wb[2] : wb[3]);
+            const int sh = (k * BITS) & 31;
+            sample((w0 >> sh) & ((1u << BITS) - 1u), (w1 >> sh) & ((1u << BITS) - 1u));
+          }
         }
       }
     }
-    x0 = nv * V;
+    constexpr uint32_t low = sizeof(T) == 1 ? 0xffu : 0xffffu;
+    m0 = sizeof(T) == 1 ? (m0 | (m0 >> 8) | (m0 >> 16) | (m0 >> 24)) & low : (m0 | (m0 >> 16)) & low;
+    m1 = sizeof(T) == 1 ? (m1 | (m1 >> 8) | (m1 >> 16) | (m1 >> 24)) & low : (m1 | (m1 >> 16)) & low;
+    x0 = head + nv * V;
   }
-  for(int x = x0 + lane; x < n; x += 32) { sample(__ldg(p0 + x), __ldg(p1 + x)); }
+  auto at = [&](int x) {
+    const uint32_t v0 = __ldg(p0 + x), v1 = __ldg(p1 + x);
+    m0 |= v0; m1 |= v1;
+    sample(v0, v1);
+  };
+  if(lane < head) { at(lane); }
+  for(int x = x0 + lane; x < n; x += 32) { at(x); }
   #pragma unroll
   for(int o = 16; o > 0; o >>= 1)
   {
     sd  += __shfl_xor_sync(kFull, sd, o);
     ssd += __shfl_xor_sync(kFull, ssd, o);
   }
-  m0_out = __reduce_max_sync(kFull, m0);
-  m1_out = __reduce_max_sync(kFull, m1);
+  m0_out = __reduce_or_sync(kFull, m0);
+  m1_out = __reduce_or_sync(kFull, m1);
   sd_out = sd;
   ssd_out = ssd;
   if(lane == 0) { a.row_ssd[warp] = ssd; }
@@ -126,8 +185,8 @@ __device__ __forceinline__ void prepass_body(const PrepassArgs& a, int block)
   {
     uint32_t m = 0;
     #pragma unroll
-    for(int w = 0; w < 8; w++) { m = max(m, s_m[lane - 6][w]); }
-    atomicMax(&o->max_sample[lane - 6], m);
+    for(int w = 0; w < 8; w++) { m |= s_m[lane - 6][w]; }
+    atomicOr(&o->or_sample[lane - 6], m);
   }
   __threadfence();                                          // the additions before the count
   __syncwarp();
@@ -192,8 +251,8 @@ __device__ __forceinline__ void prepass_totals(const PrepassArgs& a)
     else if(a.need_gcd) { g = clampi(round_half_away(ddiv((double)sd[c], area)), -a.maxdiff[c], a.maxdiff[c]); }
     o->gcd[c] = g;
   }
-  const int inv0 = __ldcg(&o->max_sample[0]) > (uint32_t)a.maxv;
-  const int inv1 = __ldcg(&o->max_sample[1]) > (uint32_t)a.maxv;
+  const int inv0 = __ldcg(&o->or_sample[0]) > (uint32_t)a.maxv;
+  const int inv1 = __ldcg(&o->or_sample[1]) > (uint32_t)a.maxv;
   const int int_path = !a.fp32_ok || ((inv0 || inv1) && !a.clip_on);
   o->flags = inv0 | (inv1 << 1) | (int_path << 2);
   o->done = 0u;
