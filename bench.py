@@ -585,8 +585,8 @@ def run_config0(ctx, steps):
 
 def run_config2(ctx, steps, hbm_peak):
     """MS-SSIM + IV-MS-SSIM of 16 blurred 2048x2048 10-bit 4:2:0 pairs per step through the batched form
-    (graphs, autotuned tiles), device frames; the moment kernels (exact sub-block moments with the next
-    scale's 2x2 downsampling fused) against the HBM bandwidth."""
+    (graphs, autotuned tiles), device frames; the window kernels (exact sub-block moments formed from the
+    pictures, with the next scales' 2x2 downsampling) against the HBM bandwidth."""
     import torch
     import qmiv_b200
     from qmiv_b200 import synth
@@ -614,15 +614,13 @@ def run_config2(ctx, steps, hbm_peak):
         ctx.set_profiling(False)
         st = ctx.stage_times(reset=True)
     mom_ms = st["ssim_win"][0] / 3
-    # algorithmic bytes of one pair's moment launches: per scale the four pictures (In0, In1 and the two
+    # algorithmic bytes of one pair's window launches: per scale the four pictures (In0, In1 and the two
     # shift-compensated pictures SCP0, SCP1) read once (scale 0: the raw 4:2:0 frames, 3 bytes per pixel,
-    # and the 16-bit 4:4:4 SCPs, 6; later scales 16-bit 4:4:4, 6 each), five uint32 moment planes per
-    # component per 4x4 block for each of the three pairs of pictures (MS-SSIM (In0, In1), IV-MS-SSIM
-    # (In0, SCP1) and (In1, SCP0): 3 x 3.75 bytes per pixel) and, below the last scale, each picture's
-    # 2x2 means (16-bit 4:4:4 at a quarter of the pixels) written once
+    # and the 16-bit 4:4:4 SCPs, 6; later scales 16-bit 4:4:4, 6 each, also written once), and the window
+    # values of the three evaluations (MS-SSIM (In0, In1), IV-MS-SSIM (In0, SCP1) and (In1, SCP0)): one double
+    # per 16 pixels, component and evaluation
     px = [w * h / 4 ** k for k in range(5)]
-    per_pair = px[0] * (3 + 3 + 6 + 6) + sum(px[k] * 4 * 6 for k in range(1, 5))
-    per_pair += sum(px[k] * 3 * 3.75 for k in range(5)) + sum(px[k] * 4 * 6 / 4 for k in range(4))
+    per_pair = px[0] * (3 + 3 + 6 + 6) + sum(px[k] * 2 * 4 * 6 for k in range(1, 5)) + sum(px[k] * 4.5 for k in range(5))
     gbs = per_pair * len(descs) / (mom_ms * 1e-3) / 1e9
     return {"value": value, "stage_ms": {k: v[0] / 3 for k, v in st.items() if v[1]},
             "moments": {"ms_per_step": mom_ms, "bytes_per_pair": per_pair, "achieved_gbs": gbs,
@@ -744,7 +742,7 @@ def run_ssim_modes(ctx, steps):
         # one window launch evaluates SSIM (In0, In1) and IV-SSIM (In0, SCP1), (In1, SCP0): 3 evaluations
         windows = 3 * ssim_option_windows(mode, window, stride)
         n = 11 if mode <= 2 else window
-        ops_per_window = n * n * (10 if mode == 0 else 5)   # float Gaussian: multiply + add per moment and tap
+        ops_per_window = n * n * 5   # one FP64 instruction per moment and tap (10-bit products are exact)
         avg_ms = win_ms / max(win_n, 1)
         achieved = windows * ops_per_window / (avg_ms * 1e-3) / 1e12
         out["options"].append({"option": name, "value": 1.0 / dt, "unit": "frame-pairs/s", "ms_per_pair": dt * 1e3,
