@@ -412,7 +412,6 @@ __global__ void __launch_bounds__(256) k_finalize(const __grid_constant__ Finali
 __global__ void __launch_bounds__(256) k_finalize_multi(const FinalizeArgs* __restrict__ pairs, const FinJob* __restrict__ jobs)
 {
   extern __shared__ double stage[];
-  wait_for_previous();
   const FinJob j = jobs[blockIdx.x];
   finalize_body(pairs[j.pair], j.chain, stage);
 }
@@ -466,7 +465,8 @@ cudaError_t launch_finalize_multi(const FinalizeArgs* d_pairs, const FinJob* d_j
   if(smem > kFinalizeMaxSmem) { return cudaErrorInvalidValue; }
   cudaError_t e = finalize_configure();
   if(e != cudaSuccess) { return e; }
-  return launch_next(k_finalize_multi, njobs, 256, smem, s, d_pairs, d_jobs);
+  k_finalize_multi<<<njobs, 256, smem, s>>>(d_pairs, d_jobs);
+  return cudaGetLastError();
 }
 
 }  // namespace qmiv

@@ -7,11 +7,12 @@
 namespace qmiv {
 
 // Launches a kernel that begins with wait_for_previous, so that its launch overlaps the end of the kernel
-// before it in the stream. Used where that paid in a whole call: the finalisers (1920x1080 88 -> 86 us,
+// before it in the stream. Used in calls of one pair where it paid: the finalisers (1920x1080 88 -> 86 us,
 // masked 4096x2048 with the mask's totals 190 -> 185) and the moment windows (4096x2048 246 -> 243). It
 // cost time before the search (four searches of a mixed batch 1464 -> 1490 us) and before the picture
 // windows and their rows (4:4:4 1920x1080 123 -> 130, eight MS-SSIM pairs 1118 -> 1185): those kernels
-// are launched plainly.
+// are launched plainly, and so are all of a batch, where it gave nothing that could be measured and the launches
+// are captured into graphs by several threads.
 template <typename... P, typename... A>
 cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args)
 {

@@ -1013,12 +1013,11 @@ static_assert(sizeof(MaskPack) <= 32000, "kernel parameters are limited to 32 KB
 template <typename T, typename TM, bool VEC>
 __global__ void __launch_bounds__(256, 2) k_mask_prepass_multi(const __grid_constant__ MaskPack pk)
 {
-  next_may_start();
   const MaskArgs& a = pk.a[blockIdx.y];
   if((int)blockIdx.x >= (VEC ? prepass420_units<TM>(a.H) : a.H)) { return; }
   if(VEC) { mask_prepass420_body<T, TM>(a, blockIdx.x); } else { mask_prepass_body<T, TM>(a, blockIdx.x); }
 }
-__global__ void k_mask_reduce_multi(const __grid_constant__ MaskPack pk) { wait_for_previous(); mask_reduce_body(pk.a[blockIdx.x]); }
+__global__ void k_mask_reduce_multi(const __grid_constant__ MaskPack pk) { mask_reduce_body(pk.a[blockIdx.x]); }
 template <typename T, typename TM, int R>
 __global__ void __launch_bounds__(256) k_cps_masked_multi(const __grid_constant__ MaskPack pk)
 {
@@ -1035,7 +1034,6 @@ __global__ void __launch_bounds__(512, 2) k_cps_masked_key_multi(const __grid_co
 }
 __global__ void __launch_bounds__(256) k_mask_finalize_multi(const __grid_constant__ MaskPack pk)
 {
-  wait_for_previous();
   mask_finalize_body(pk.a[blockIdx.x / 9], blockIdx.x % 9);
 }
 
@@ -1550,7 +1548,7 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
   }
   clock_.end(s, QMIV_STAGE_PREPASS, tok);
   tok = clock_.begin(ctx, s);
-  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); QMIV_CUDA(launch_next(k_mask_reduce_multi, cnt, 32, 0, s, pk)); }
+  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); k_mask_reduce_multi<<<cnt, 32, 0, s>>>(pk); }
   clock_.end(s, QMIV_STAGE_REDUCE, tok);
   tok = clock_.begin(ctx, s);
   for(auto& g : srch)
@@ -1575,7 +1573,7 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
   }
   clock_.end(s, QMIV_STAGE_CPS, tok);
   tok = clock_.begin(ctx, s);
-  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); QMIV_CUDA(launch_next(k_mask_finalize_multi, 9 * cnt, 256, 0, s, pk)); }
+  for(size_t f = 0; f < all.size(); f += kPackPairs) { const int cnt = pack(all, f); k_mask_finalize_multi<<<9 * cnt, 256, 0, s>>>(pk); }
   clock_.end(s, QMIV_STAGE_FINALIZE, tok);
   QMIV_CUDA(cudaGetLastError());
   tok = clock_.begin(ctx, s);
