@@ -23,6 +23,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 namespace qmiv {
 
@@ -193,8 +194,19 @@ Engine::~Engine()
   if(stream_) { cudaStreamDestroy(stream_); }
 }
 
+// Capture, instantiation, launch and destruction of graphs take turns over all engines. Two server workers that
+// did these at the same time crashed inside cuGraphLaunch in 2 of 13 runs of a four-second request stream
+// (driver 580.159); each engine uses only its own graphs, so the calls alone meet in the driver. A launch holds
+// the lock for some 10 us of host time.
+static std::mutex& graph_mutex()
+{
+  static std::mutex mu;
+  return mu;
+}
+
 void Engine::clear_graphs()
 {
+  std::lock_guard<std::mutex> lk(graph_mutex());
   for(auto& g : graphs_) { if(g.second) { cudaGraphExecDestroy(g.second); } }
   graphs_.clear();
 }
@@ -457,6 +469,7 @@ qmiv_status Engine::submit(const qmiv_pair_desc* pairs, int32_t n)
   };
   if(graph)
   {
+    std::lock_guard<std::mutex> lk(graph_mutex());
     cudaGraphExec_t& ex = graphs_[sig];
     if(!ex)
     {
