@@ -79,6 +79,11 @@ _RESULT, _RESULT_FIELDS = _result_layout()
 assert _RESULT.size == ctypes.sizeof(QmivResult)
 
 
+class QmivCpsKeys(ctypes.Structure):
+    _fields_ = [("shared", ctypes.c_int32), ("masked", ctypes.c_int32), ("key_bits", ctypes.c_int32), ("mid", ctypes.c_int32),
+                ("bias", ctypes.c_uint32), ("masked_value", ctypes.c_uint32), ("sum_split", ctypes.c_int32)]
+
+
 class QmivPairDesc(ctypes.Structure):
     _fields_ = [("in0", QmivFrame), ("in1", QmivFrame), ("width", ctypes.c_int32), ("height", ctypes.c_int32),
                 ("bitdepth", ctypes.c_int32), ("chroma_format", ctypes.c_int32), ("search_range", ctypes.c_int32),
@@ -142,6 +147,8 @@ SIGNATURES = {
     "qmiv_probe_int32_peak": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(ctypes.c_double)]),
     "qmiv_probe_fp32_peak": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(ctypes.c_double)]),
     "qmiv_probe_fp64_peak": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(ctypes.c_double)]),
+    "qmiv_probe_cps_keys": (ctypes.c_int, [ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32),
+                                           ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(QmivCpsKeys)]),
     "qmiv_batch_destroy": (ctypes.c_int, [_P]),
     "qmiv_batch_stream": (ctypes.c_int, [_P, _PP]),
     "qmiv_batch_compute": (ctypes.c_int, [_P, ctypes.POINTER(QmivPairDesc), ctypes.c_int32, ctypes.POINTER(QmivResult)]),

@@ -60,9 +60,6 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// K = 2^key_bits: above the largest raster index
-__host__ __device__ constexpr int key_bits(int R) { return R <= 2 ? 5 : (R == 3 ? 6 : 7); }
-
 // Sample type of the mask of a search without one
 struct NoMask { };
 
@@ -72,7 +69,7 @@ struct Geo420
 {
   static constexpr bool MASK = !std::is_same<TM, NoMask>::value;
   static constexpr int D = 2 * R + 1;
-  static constexpr int KB = key_bits(R);                           // key bits of the raster code
+  static constexpr int KB = cps_key_bits(R);                           // key bits of the raster code
   static constexpr uint32_t K = 1u << KB;
   static_assert(D * D <= (1 << KB), "raster codes fit");
   static constexpr int TW = 128, TH = 16, NT = 256;
@@ -615,8 +612,7 @@ __device__ __forceinline__ void epilogue420(const CpsArgs& a, const unsigned cha
 }
 
 // Epilogue of a masked search: squared differences weighted by the test pixels' mask values, summed per row in
-// 64 bits. A row's four terms are below 2^40 (differences below 2^13, mask values below 2^14); over the
-// warp the parts from bit 13 up (< 2^27 each) and the low 13 bits are summed in 32 bits.
+// 64 bits, over the warp as two 32-bit parts (kMaskSumSplit).
 template <int R, typename T, typename TM>
 __device__ __forceinline__ void epilogue420_masked(const CpsArgs& a, const unsigned char* ref, const TM* mask, const uint32_t* off, uint32_t base,
                                                    const uint32_t ty[16], const uint32_t tu[4], const uint32_t tv[4],
@@ -652,11 +648,12 @@ __device__ __forceinline__ void epilogue420_masked(const CpsArgs& a, const unsig
     #pragma unroll
     for(int c = 0; c < 3; c++)
     {
-      const uint32_t h = __reduce_add_sync(kFull, (uint32_t)(rs[c] >> 13)), l = __reduce_add_sync(kFull, (uint32_t)rs[c] & 0x1fffu);
+      const uint32_t h = __reduce_add_sync(kFull, (uint32_t)(rs[c] >> kMaskSumSplit));
+      const uint32_t l = __reduce_add_sync(kFull, (uint32_t)rs[c] & ((1u << kMaskSumSplit) - 1u));
       if(lane == 3 * i + c) { hi = h; lo = l; }
     }
   }
-  const uint64_t sum = ((uint64_t)hi << 13) + lo;
+  const uint64_t sum = ((uint64_t)hi << kMaskSumSplit) + lo;
   if(lane < 12 && yb + lane / 3 < a.H && sum != 0) { atomicAdd(rows + (size_t)yb * 3 + lane, (unsigned long long)sum); }
 }
 
@@ -943,7 +940,7 @@ bool cps_shared_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[
 {
   const int64_t m = ((int64_t)maxv + 1) / 2;
   const int D = 2 * R + 1;
-  const int64_t K = (int64_t)1 << key_bits(R);
+  const int64_t K = (int64_t)1 << cps_key_bits(R);
   long double lo = 0, hi = 0;
   for(int c = 0; c < 3; c++)
   {
@@ -959,12 +956,12 @@ bool cps_shared_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[
 }
 
 // Masked search: a masked sample's keys, masked + P + code, must lie above every real key and below 2^32.
-// P lies between K w_0 (mid + g_0)^2 and K (lo + hi_1 + hi_2), with lo and hi as above; the row sums need
-// differences below 2^13.
+// P lies between K w_0 (mid + g_0)^2 and K (lo + hi_1 + hi_2), with lo and hi as above; the row sums' split
+// (kMaskSumSplit) needs differences below 2^13.
 bool cps_masked_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[3], uint32_t* masked)
 {
   if(!cps_shared_key(R, maxv, w, gmax, nullptr, nullptr)) { return false; }
-  const int64_t m = ((int64_t)maxv + 1) / 2, D = 2 * R + 1, K = (int64_t)1 << key_bits(R), code = (3 + 2 * R) * D + 3 + 2 * R;
+  const int64_t m = ((int64_t)maxv + 1) / 2, D = 2 * R + 1, K = (int64_t)1 << cps_key_bits(R), code = (3 + 2 * R) * D + 3 + 2 * R;
   int64_t lo = 0, hi = 0, hic = 0;   // bounded by cps_shared_key
   bool small = true;
   for(int c = 0; c < 3; c++)

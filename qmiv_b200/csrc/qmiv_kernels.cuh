@@ -301,6 +301,11 @@ bool cps_fp32_exact(int32_t maxv, const int32_t w[3], const int32_t maxdiff[3]);
 bool cps_shared_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[3], uint32_t* bias, int32_t* mid);
 // ... and for its masked search.
 bool cps_masked_key(int R, int32_t maxv, const int32_t w[3], const int32_t gmax[3], uint32_t* masked);
+// Bits of a key below the error: 2^bits lies above the largest raster index.
+__host__ __device__ constexpr int cps_key_bits(int R) { return R <= 2 ? 5 : (R == 3 ? 6 : 7); }
+// Masked row sums: a lane's four terms d^2 M of a row are below 2^44 (cps_masked_key: |d| < 2^13; any 16-bit M);
+// over a warp their parts below and from this bit up, below 2^22 each, are summed apart in 32 bits.
+constexpr int kMaskSumSplit = 22;
 // ... for the form a picture of these chroma shifts is searched with.
 bool cps_key_exact(int R, int sx, int sy, int32_t maxv, const int32_t w[3], const int32_t maxdiff[3]);
 // Tile form 1 is the 4:2:0 form; the others are the warps of a tile column.

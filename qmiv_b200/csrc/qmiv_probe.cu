@@ -144,4 +144,19 @@ qmiv_status qmiv_probe_fp64_peak(int32_t device, int32_t iters, double* tops)
   return QMIV_OK;
 }
 
+qmiv_status qmiv_probe_cps_keys(int32_t search_range, int32_t max_sample, const int32_t weights[3], const int32_t gcd_bound[3],
+                                qmiv_cps_keys* out)
+{
+  if(!weights || !gcd_bound || !out || search_range < 1 || search_range > 5 || max_sample < 1 || max_sample > 65535)
+  {
+    return fail(QMIV_ERR_INVALID_ARG, "bad probe arguments");
+  }
+  *out = qmiv_cps_keys{};
+  out->shared = cps_shared_key(search_range, max_sample, weights, gcd_bound, &out->bias, &out->mid) ? 1 : 0;
+  out->masked = cps_masked_key(search_range, max_sample, weights, gcd_bound, &out->masked_value) ? 1 : 0;
+  out->key_bits = cps_key_bits(search_range);
+  out->sum_split = kMaskSumSplit;
+  return QMIV_OK;
+}
+
 }  // extern "C"
