@@ -493,21 +493,22 @@ __device__ __forceinline__ void ssim_rows_body(const SsimRowJob& J, int band)
 
 // Every kernel takes its jobs by value (one pair) or from a table in device memory. The job is the fastest
 // grid dimension of the picture kernels, so that the evaluations that share a picture read its tiles close
-// together in time.
+// together in time, and of every table kernel: a pair has up to 54 jobs, and only the first grid dimension goes
+// past 65535.
 __device__ __forceinline__ void ssim_win_any(const SsimPoolJob& J, int tile_x, int band)
 {
   __shared__ __align__(16) uint32_t st[5][kStRows][kStCols];
   ssim_win_body(J, st, tile_x, band);
 }
 __global__ void __launch_bounds__(kWinNT, kWinOcc) k_ssim_win(const __grid_constant__ JobArgs<SsimPoolJob, kMaxPoolJobs> a) { wait_for_previous(); ssim_win_any(a.job[blockIdx.z], blockIdx.x, blockIdx.y); }
-__global__ void __launch_bounds__(kWinNT, kWinOcc) k_ssim_win_multi(const SsimPoolJob* __restrict__ jobs) { ssim_win_any(jobs[blockIdx.z], blockIdx.x, blockIdx.y); }
+__global__ void __launch_bounds__(kWinNT, kWinOcc) k_ssim_win_multi(const SsimPoolJob* __restrict__ jobs) { ssim_win_any(jobs[blockIdx.x], blockIdx.y, blockIdx.z); }
 template <int N>
 __global__ void __launch_bounds__(kWinNT, kImgOcc) k_ssim_img(const __grid_constant__ JobArgs<SsimImgJob, N> a) { ssim_img_any(a.job[blockIdx.x], blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(kWinNT, kImgOcc) k_ssim_img_multi(const SsimImgJob* __restrict__ jobs) { ssim_img_any(jobs[blockIdx.x], blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(256) k_ssim_pyr(const __grid_constant__ JobArgs<SsimPyrJob, kMaxPyrJobs> a) { ssim_pyr_any(a.job[blockIdx.z], blockIdx.x, blockIdx.y); }
-__global__ void __launch_bounds__(256) k_ssim_pyr_multi(const SsimPyrJob* __restrict__ jobs) { ssim_pyr_any(jobs[blockIdx.z], blockIdx.x, blockIdx.y); }
+__global__ void __launch_bounds__(256) k_ssim_pyr_multi(const SsimPyrJob* __restrict__ jobs) { ssim_pyr_any(jobs[blockIdx.x], blockIdx.y, blockIdx.z); }
 __global__ void __launch_bounds__(32 * kRowWarps, 3) k_ssim_rows(const __grid_constant__ JobArgs<SsimRowJob, kMaxRowJobs> a) { next_may_start(); ssim_rows_body(a.job[blockIdx.y], blockIdx.x); }
-__global__ void __launch_bounds__(32 * kRowWarps, 3) k_ssim_rows_multi(const SsimRowJob* __restrict__ jobs) { ssim_rows_body(jobs[blockIdx.y], blockIdx.x); }
+__global__ void __launch_bounds__(32 * kRowWarps, 3) k_ssim_rows_multi(const SsimRowJob* __restrict__ jobs) { ssim_rows_body(jobs[blockIdx.x], blockIdx.y); }
 
 // ---- host ---------------------------------------------------------------------------------------
 static int tiles_of(int nx) { return (nx + kWinX - 1) / kWinX; }
@@ -664,12 +665,12 @@ cudaError_t launch_ssim_tables(const SsimTables& t, cudaStream_t s, bool rows_on
   cudaError_t e = cudaSuccess;
   if(rows_only)
   {
-    if(t.nrows) { k_ssim_rows_multi<<<dim3(bands_of(d.rows_ny), t.nrows), 32 * kRowWarps, 0, s>>>(t.rows); e = last_or(e); }
+    if(t.nrows) { k_ssim_rows_multi<<<dim3(t.nrows, bands_of(d.rows_ny)), 32 * kRowWarps, 0, s>>>(t.rows); e = last_or(e); }
     return e;
   }
-  if(t.npool) { k_ssim_win_multi<<<dim3(tiles_of(d.pool_nx), bands_of(d.pool_ny), t.npool), kWinNT, 0, s>>>(t.pool); e = last_or(e); }
+  if(t.npool) { k_ssim_win_multi<<<dim3(t.npool, tiles_of(d.pool_nx), bands_of(d.pool_ny)), kWinNT, 0, s>>>(t.pool); e = last_or(e); }
   if(t.nimg0) { k_ssim_img_multi<<<dim3(t.nimg0, tiles_of(d.img0_nx), bands_of(d.img0_ny)), kWinNT, 0, s>>>(t.img0); e = last_or(e); }
-  if(t.npyr) { k_ssim_pyr_multi<<<dim3((d.pyr_w + 2 * kPyrW - 1) / (2 * kPyrW), (d.pyr_h + 2 * kPyrH - 1) / (2 * kPyrH), t.npyr), 256, 0, s>>>(t.pyr); e = last_or(e); }
+  if(t.npyr) { k_ssim_pyr_multi<<<dim3(t.npyr, (d.pyr_w + 2 * kPyrW - 1) / (2 * kPyrW), (d.pyr_h + 2 * kPyrH - 1) / (2 * kPyrH)), 256, 0, s>>>(t.pyr); e = last_or(e); }
   if(t.nimgn) { k_ssim_img_multi<<<dim3(t.nimgn, tiles_of(d.imgn_nx), bands_of(d.imgn_ny)), kWinNT, 0, s>>>(t.imgn); e = last_or(e); }
   return e;
 }

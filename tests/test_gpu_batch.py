@@ -169,3 +169,18 @@ def test_batch_submit_wait_two_in_flight(qctx):
         with pytest.raises(qmiv_b200.QmivError):
             batch.wait(ta)
         ta = batch.submit(da)   # left in flight: destroying the batch waits for it
+
+
+@pytest.mark.parametrize("size,metrics,n", [(64, ALL_METRICS, 2500), (128, ["MSSSIM", "IVMSSSIM"], 5600)])
+def test_batch_of_many_small_pairs(size, metrics, n, qctx):
+    """More than 65535 window-row jobs (27 a pair here) and, in the larger set, as many plane pyramids (12 a pair) in
+    one call: the same results as a small batch's."""
+    import qmiv_b200
+    spec = (size, size, 8, 420, 1, metrics)
+    base = [_frames(spec, seed, device=True) for seed in range(3)]
+    pairs = [dict(frame0=base[i % 3][0], frame1=base[i % 3][1], width=size, height=size, bitdepth=8, search_range=1, metrics=metrics)
+             for i in range(n)]
+    with qmiv_b200.Batch(qctx, n, n * size * size) as b:
+        few = b.compute(pairs[:3])
+        many = b.compute(pairs)
+    assert all(many[i] == few[i % 3] for i in range(n))
