@@ -1,6 +1,6 @@
 // Corresponding-pixel-shift search (libs/pmbb-ivqm/src/xCorrespPixelShiftSSE.cpp:18-127) of 4:2:2 and
 // 4:4:4 pictures for sm_100a: persistent CTAs, TMA tile loads, 4 x 2 pixels per thread in the search.
-// (4:2:0: qmiv_cps420.cu.)
+// (4:2:0: qmiv_cps420.cuh.)
 //
 // Per tile of 128 x TH output pixels (TH = 32, or 16 when shared memory is short or the autotuner
 // prefers two CTAs per SM) a CTA of 2 x TH / 4 warps
@@ -881,7 +881,7 @@ cudaError_t launch_cps_multi(const void* d_descs, const int32_t* d_prefix, int n
   cudaError_t e = cudaGetDevice(&dev);
   if(e != cudaSuccess) { return e; }
   const CpsKernelArgs* d = static_cast<const CpsKernelArgs*>(d_descs);
-  if(wy == kCpsForm420) { return cps420_launch_multi(d, d_prefix, npairs, ntiles, R, esz, 0, s); }
+  if(wy == kCpsForm420) { return cps420_launch_multi(d, d_prefix, ntiles, R, esz, s); }
   auto go = [&](auto tag) -> cudaError_t {
     using T = decltype(tag);
     switch(R)

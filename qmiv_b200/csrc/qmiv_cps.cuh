@@ -1,6 +1,6 @@
 // Pieces shared by the two forms of the corresponding-pixel-shift search: the work-list descriptor,
 // TMA tile loads with bounded waits, tensor-map encoding and launch helpers (qmiv_cps.cu: any chroma
-// format; qmiv_cps420.cu: 4:2:0).
+// format; qmiv_cps420.cuh: 4:2:0).
 #pragma once
 #include "qmiv_kernels.cuh"
 
@@ -133,11 +133,11 @@ int grid_for(F* fn, int threads, size_t smem, int ntiles, int dev)
 constexpr int kAlign = 128;
 __host__ __device__ constexpr uint32_t align_up(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
 
-// ---- the 4:2:0 form (qmiv_cps420.cu) ----------------------------------------------------------
+// ---- the 4:2:0 form (qmiv_cps420.cuh) ----------------------------------------------------------
 bool        cps420_fits(int R, int esz);
 int         cps420_tiles(int W, int H);
 cudaError_t cps420_describe(CpsKernelArgs& k, int R, int esz, CpsPairPlan* plan);
 cudaError_t cps420_launch(const CpsKernelArgs& k, int R, int esz, cudaStream_t s);
-cudaError_t cps420_launch_multi(const CpsKernelArgs* d, const int32_t* prefix, int npairs, int ntiles, int R, int esz, int mesz, cudaStream_t s);
+cudaError_t cps420_launch_multi(const CpsKernelArgs* d, const int32_t* prefix, int ntiles, int R, int esz, cudaStream_t s);
 
 }  // namespace qmiv

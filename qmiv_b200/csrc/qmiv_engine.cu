@@ -194,10 +194,12 @@ Engine::~Engine()
   if(stream_) { cudaStreamDestroy(stream_); }
 }
 
-// Capture, instantiation, launch and destruction of graphs take turns over all engines. Two server workers that
-// did these at the same time crashed inside cuGraphLaunch in 2 of 13 runs of a four-second request stream
-// (driver 580.159); each engine uses only its own graphs, so the calls alone meet in the driver. A launch holds
-// the lock for some 10 us of host time.
+// Capture, instantiation, launch and destruction of graphs take turns over all engines: a precaution, not a
+// proven mend. Two server workers that did these at the same time crashed inside cuGraphLaunch in 2 of 13 runs of
+// a four-second request stream (driver 580.159). Each engine uses its own graphs alone, drops them before a buffer
+// that they name is freed or moved, and never does so with a call in flight, so nothing in this file explains it.
+// Since then a captured search takes pointers alone (its kernel had an argument block of 1.2 KB, 64-byte
+// aligned, by value) and the server's engines replay no graphs. A launch holds the lock for some 10 us of host time.
 static std::mutex& graph_mutex()
 {
   static std::mutex mu;

@@ -293,7 +293,7 @@ cudaError_t launch_cps_multi(const void* d_descs, const int32_t* d_prefix, int n
 
 // The masked search of 4:2:0 pictures (CpsArgs::mask set) for one pair, and for a work list of described pairs
 cudaError_t launch_cps_masked420(const CpsArgs& a, int R, int esz, cudaStream_t s);
-cudaError_t launch_cps_masked420_multi(const void* d_descs, const int32_t* d_prefix, int npairs, int ntiles, int R, int esz, int mesz, cudaStream_t s);
+cudaError_t launch_cps_masked420_multi(const void* d_descs, const int32_t* d_prefix, int ntiles, int R, int esz, int mesz, cudaStream_t s);
 
 // Exactness check of the fp32 key path for a given bit depth, weights and GCD clip range.
 bool cps_fp32_exact(int32_t maxv, const int32_t w[3], const int32_t maxdiff[3]);

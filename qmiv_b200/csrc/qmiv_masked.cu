@@ -14,7 +14,7 @@
 //                    are weighted by the test pixel's mask value and summed per row in uint64;
 //                    k_cps_masked_key is the same search by exact fp32 keys, both directions per
 //                    CTA, four pixels per thread, where the bit depth, weights and GCD range bound
-//                    every error; 4:2:0 pictures take the integer-key search of qmiv_cps420.cu
+//                    every error; 4:2:0 pictures take the integer-key search of qmiv_cps420.cuh
 //   k_mask_finalize  the ordered compensated sums (xKBNS.h:36-43) of the ERP row weights and the
 //                    row totals, one CTA per chain (terms staged in shared memory, one thread sums)
 // dB values, exact-component fake values and the picture averages are formed on the host in
@@ -79,7 +79,7 @@ struct MaskPlan
   size_t              mesz = 1;      // bytes per mask sample
   int32_t             maxdiff[4] = { 0, 0, 0, 0 };
   bool                key = false;   // the exact-key search applies (k_cps_masked_key)
-  bool                key420 = false;   // the 4:2:0 integer-key search applies (qmiv_cps420.cu)
+  bool                key420 = false;   // the 4:2:0 integer-key search applies (qmiv_cps420.cuh)
   double              ws_corr = 1.0;
   std::vector<double> ws;            // [H] with ERP
 };
@@ -1558,7 +1558,7 @@ qmiv_status MaskedBatch::run(qmiv_ctx_s* ctx, const qmiv_params& prm0, cudaStrea
     if(std::get<3>(g.first) == 2)
     {
       const List& L = lists[g.first];
-      const cudaError_t e = launch_cps_masked420_multi(L.desc, L.prefix, (int)g.second.pairs.size(), L.tiles, R, t, tm, s);
+      const cudaError_t e = launch_cps_masked420_multi(L.desc, L.prefix, L.tiles, R, t, tm, s);
       if(e != cudaSuccess) { return cuda_fail(e, "masked search launch"); }
       continue;
     }

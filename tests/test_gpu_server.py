@@ -109,3 +109,20 @@ def test_server_waits_and_timeouts(qctx):
         pending = [srv.submit(fr, 256, 128, 10, metrics=["IVPSNR"]) for _ in range(3)]
     # destroy waited for the pending requests; their tickets are gone with the server
     assert len(pending) == 3
+
+
+def test_workers_repeat_signatures(qctx):
+    """Several workers run batches of the same signatures over and over at the same time (each signature often
+    enough to be captured, were it replayed from graphs): every result equals the one-pair form's."""
+    import qmiv_b200
+    shapes = [(256, 128, 10, 2, "IVPSNR,IVSSIM"), (192, 96, 8, 3, "PSNR,IVPSNR")]
+    frames = [_req_frames(W, H, bd, 2, 40 + k, device=True) for k, (W, H, bd, R, m) in enumerate(shapes)]
+    plain = []
+    for (W, H, bd, R, m), fr in zip(shapes, frames):
+        with qmiv_b200.Calc(qctx, W, H, bd, search_range=R) as calc:
+            plain.append([calc.compute(a, b, qmiv_b200.metric_mask(m)) for a, b in fr])
+    with qmiv_b200.Server(qctx, max_batch_pairs=2, max_batch_pixels=2 * 256 * 128, workers=4) as srv:
+        tickets = [(k, srv.submit(frames[k], *shapes[k][:3], search_range=shapes[k][3], metrics=shapes[k][4]))
+                   for _ in range(60) for k in range(len(shapes))]
+        for k, t in tickets:
+            assert srv.wait(t)[0] == plain[k]
