@@ -96,12 +96,14 @@ struct Geo420
   static constexpr int CPP = CW / 2;                               // chroma
   static_assert(CW % 2 == 0, "whole chroma pairs");
   static constexpr uint32_t LUMA = (uint32_t)SH * LPP * 16u, CHROMA = (uint32_t)CH * CPP * 16u;   // per picture
-  // Three CTAs per SM where they fit with one raw stage each (R <= 2), else two (one at R = 5) with the
-  // raw boxes double-buffered.
-  static constexpr uint32_t TILES = 2 * LUMA + 2 * CHROMA + kAlign + 32;
-  static constexpr int CTAS = 3 * (TILES + STAGE + 3584u) <= 227u * 1024u ? 3 : (R <= 4 ? 2 : 1);
-  static constexpr uint32_t STAGES = CTAS == 3 ? 1 : 2;
+  // Three CTAs per SM where they fit with one raw stage each (R <= 2, R = 3 with bytes), else two (unmasked one at
+  // R = 5), with the raw boxes double-buffered where as many CTAs still fit. With a mask, full, 4096x2048 10 bits: one
+  // CTA was resident with two stages, 372 us a call at R = 4 and 536 at R = 5; two with one stage take 296 and 408.
+  static constexpr uint32_t TILES = 2 * LUMA + 2 * CHROMA + kAlign + 32, PER_SM = 227u * 1024u, FIXED = 3584u;   // static and reserved
+  static constexpr int CTAS = 3 * (TILES + STAGE + FIXED) <= PER_SM ? 3 : (R <= 4 || MASK ? 2 : 1);
+  static constexpr uint32_t STAGES = CTAS < 3 && CTAS * (TILES + 2 * STAGE + FIXED) <= PER_SM ? 2 : 1;
   static constexpr uint32_t SMEM = TILES + STAGES * STAGE;
+  static_assert(CTAS * (SMEM + FIXED) <= PER_SM, "the CTAs that the registers are shared out for are resident");
   // a thread's window: luma samples and chroma samples across / down
   static constexpr int WL = 4 + 2 * R, WC = ((3 + 2 * R + ODD) >> 1) + 1;
   static_assert(WL % 2 == 0 && WC % 2 == 0, "windows of whole pairs");
