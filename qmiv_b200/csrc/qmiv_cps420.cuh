@@ -43,9 +43,14 @@
 // are double-buffered only where three CTAs do not fit.
 //
 // With a mask (mask mode) the same tiles also bring the mask's samples; masked reference samples are staged
-// above every real key and the winners' squared differences are weighted by the test pixels' mask values.
-// 4096x2048, 10 bits, 8-bit mask: 193 us by the fp32-key kernel (one pixel column per thread, tiles staged
-// sample by sample, no copies in flight) -> 115; 8 pairs of 1920x1080, 8 bits: 383 -> 244.
+// above every real key and the winners' squared differences are weighted by the test pixels' mask values. A strip of
+// 128 x 4 pixels without a kept one is not searched, a tile without one not staged. Calls of 4096x2048, 10 bits,
+// 8-bit mask, R = 2: full mask 290 us by the fp32-key kernel (one pixel column per thread, tiles staged sample by sample, no
+// copies in flight) -> 162, a disc (31 % of the picture) 214 -> 113, a rectangle of 5 % 184 -> 89; R = 4 452 -> 296,
+// 270 -> 163, 197 -> 100. Where single 16x16 blocks are strewn over the picture, 20 % of them kept, the strips of
+// 32 x 4 pixels of that kernel left out more: 219 -> 156 at R = 2, 280 -> 287 at R = 4, 367 -> 405 at R = 5. Dealing the
+// kept 4x4 blocks to as few warps as hold them took longer still (424 at R = 4): a tile lasts as long as one warp.
+// 8 pairs of 1920x1080, 8 bits, 60 % of the 16x16 blocks kept: 729 -> 402.
 //
 // Pictures with samples above the maximum (SKIP and WARN actions) and parameters whose keys do not fit
 // take the literal int32 search below (the SSE path's wrap-around arithmetic) in the same frame.
@@ -274,6 +279,31 @@ __device__ __forceinline__ void load4(const T* p, uint32_t v[4])
     #pragma unroll
     for(int k = 0; k < 4; k++) { v[k] = p[k]; }
   }
+}
+
+// Bit q: the mask keeps a sample in the tile's rows 4 q .. 4 q + 3 (128 columns; past the picture the box holds anything,
+// so a bit too many there). The same for every warp, which reads the whole tile: 16 bytes a lane and load.
+template <int R, typename T, typename TM>
+__device__ __forceinline__ uint32_t kept_strips(const unsigned char* raw, int lane)
+{
+  using G = Geo420<R, T, TM>;
+  constexpr int PER_ROW = G::TW * G::MESZ / 16, ROWS = 32 / PER_ROW;   // lanes of a row, rows of a load
+  static_assert(4 % ROWS == 0 && G::AXM * G::MESZ == 16 && G::BWM * G::MESZ % 16 == 0 && G::OFFM % 16 == 0, "aligned loads");
+  const unsigned char* p = raw + G::OFFM + (R + lane / PER_ROW) * (G::BWM * G::MESZ) + 16 + 16 * (lane % PER_ROW);
+  uint32_t bits = 0;
+  #pragma unroll
+  for(int q = 0; q < 4; q++)
+  {
+    uint32_t any = 0;
+    #pragma unroll
+    for(int r = 4 * q; r < 4 * q + 4; r += ROWS)
+    {
+      const uint4 v = *reinterpret_cast<const uint4*>(p + r * (G::BWM * G::MESZ));
+      any |= v.x | v.y | v.z | v.w;
+    }
+    bits |= __any_sync(kFull, any != 0u) ? 1u << q : 0u;
+  }
+  return bits;
 }
 
 // Test samples of the 4x4 block at (block row by, block column lane): 16 luma, 2x2 of either chroma.
@@ -751,71 +781,88 @@ __device__ __forceinline__ void cps420_body(const CpsKernelArgs* descs, const in
     const bool clip = a.clip < (sizeof(T) == 1 ? 0xffu : 0xffffu);
     const bool border = x0 < R || y0 < R || x0 + G::TW + R > a.W || y0 + G::TH + R > a.H;
     if(clip || border) { complete_halo<R, T, TM>(a, box, x0, y0, clip, border); }
+    const int xb = x0 + 4 * lane, yb = y0 + 4 * by;
+    bool kept = true;
+    if constexpr(G::MASK)
+    {
+      // A pixel with M = 0 adds nothing: a warp without another in its strip skips search and epilogue, a tile
+      // without another is done.
+      const uint32_t strips = kept_strips<R, T, TM>(box, lane);
+      kept = (strips >> by) & 1u;
+      if(strips == 0u)                                      // the same for every warp
+      {
+        if(G::STAGES == 1) { __syncthreads(); }             // the one raw stage has been read
+        issue_next(t + (int)gridDim.x, G::STAGES == 2 ? stage ^ 1u : 0u);
+        continue;
+      }
+    }
     const uint32_t kw0 = G::K * (uint32_t)a.wi[0], kw1 = G::K * (uint32_t)a.wi[1], kw2 = G::K * (uint32_t)a.wi[2];
     const int32_t mid = a.key_mid;
     stage420<R, T, TM>(box, luma, chroma, kw0, kw1, kw2, G::K * a.key_bias, mid, a.key_masked);
     __syncthreads();
     if(G::STAGES == 2) { issue_next(t + (int)gridDim.x, stage ^ 1u); }
-    // dir 0 (R2T): test = In0 + GCD searched in In1 -> rows[0], SCP1 = clip(In1[best] - GCD)
-    // dir 1 (T2R): test = In1 - GCD searched in In0 -> rows[1], SCP0 = clip(In0[best] + GCD)
-    const int sg = dir ? -1 : 1;
-    const int g0 = sg * s_gcd[0], g1 = sg * s_gcd[1], g2 = sg * s_gcd[2];
-    const unsigned char* tst = box + dir * G::PIC;
-    const unsigned char* ref = box + (dir ^ 1) * G::PIC;
-    uint32_t idx[16];
-    const int lofs = 4 * by * G::BWL + (G::AX - R) + 4 * lane, cofs = 2 * by * G::BWC + (G::AX - G::CR0) + 2 * lane;
-    if(G::MASK || (s_gcd[3] & 4) == 0)
+    if(!G::MASK || kept)
     {
-      uint32_t c0[16], c1[4], c2[4], ty[16], tu[4], tv[4];
-      load_test420<R, T>(tst, by, lane, 0, ty, tu, tv);
-      const uint32_t m0 = 0u - 2u * kw0, m1 = 0u - 2u * kw1, m2 = 0u - 2u * kw2;
-      const uint32_t o0 = m0 * (uint32_t)(g0 - mid), o1 = m1 * (uint32_t)(g1 - mid), o2 = m2 * (uint32_t)(g2 - mid);
-      #pragma unroll
-      for(int p = 0; p < 16; p++) { c0[p] = m0 * ty[p] + o0; }
-      #pragma unroll
-      for(int b = 0; b < 4; b++) { c1[b] = m1 * tu[b] + o1; c2[b] = m2 * tv[b] + o2; }
-      // held in registers from here on: recomputed from the test samples at every use they would
-      // cost the search as many multiply-adds again
-      #pragma unroll
-      for(int p = 0; p < 16; p++) { asm volatile("" : "+r"(c0[p])); }
-      #pragma unroll
-      for(int b = 0; b < 4; b++) { asm volatile("" : "+r"(c1[b]), "+r"(c2[b])); }
-      search420<R, T>(luma + (dir ^ 1) * (G::SH * G::LPP) + 4 * by * G::LPP + lane,
-                      chroma + (dir ^ 1) * (G::CH * G::CPP) + 2 * by * G::CPP + lane, c0, c1, c2, idx);
-    }
-    else
-    {
-      uint32_t found[16];
-      search420_literal<R, T>(tst, ref, lofs, cofs, (uint32_t)a.wi[0], (uint32_t)a.wi[1], (uint32_t)a.wi[2], g0, g1, g2, found);
-      #pragma unroll
-      for(int p = 0; p < 16; p++) { idx[p] = found[p]; }
-    }
-    // the test samples are read again: kept through the search they would take 24 registers from it
-    uint32_t ty[16], tu[4], tv[4];
-    int zero = 0;
-    asm volatile("" : "+r"(zero));
-    load_test420<R, T>(tst, by, lane, zero, ty, tu, tv);
-    const uint32_t base = (uint32_t)(lofs * G::ESZ) | ((uint32_t)(cofs * G::ESZ) << 16);
-    const int xb = x0 + 4 * lane, yb = y0 + 4 * by;
-    if constexpr(G::MASK)
-    {
-      epilogue420_masked<R, T, TM>(a, ref, reinterpret_cast<const TM*>(box + G::OFFM) + (4 * by + R) * G::BWM + G::AXM + 4 * lane, s_off, base, ty, tu,
-                                   tv, idx, dir, xb, yb, g0, g1, g2);
-    }
-    else
-    {
-    const int sel = ((x0 + G::TW > a.W || y0 + G::TH > a.H) ? 4 : 0) | (a.mom[dir].p != nullptr ? 2 : 0) |
-                    ((dir ? a.scp0 : a.scp1) != nullptr ? 1 : 0);
-    switch(sel)
-    {
-    case 0: epilogue420<R, T, false, false, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
-    case 1: epilogue420<R, T, false, false, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
-    case 2: epilogue420<R, T, false, true, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
-    case 4: epilogue420<R, T, true, false, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
-    case 6: epilogue420<R, T, true, true, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
-    case 5: epilogue420<R, T, true, false, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
-    default: epilogue420<R, T, true, true, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;   // 3, 7
-    }
+      // dir 0 (R2T): test = In0 + GCD searched in In1 -> rows[0], SCP1 = clip(In1[best] - GCD)
+      // dir 1 (T2R): test = In1 - GCD searched in In0 -> rows[1], SCP0 = clip(In0[best] + GCD)
+      const int sg = dir ? -1 : 1;
+      const int g0 = sg * s_gcd[0], g1 = sg * s_gcd[1], g2 = sg * s_gcd[2];
+      const unsigned char* tst = box + dir * G::PIC;
+      const unsigned char* ref = box + (dir ^ 1) * G::PIC;
+      uint32_t idx[16];
+      const int lofs = 4 * by * G::BWL + (G::AX - R) + 4 * lane, cofs = 2 * by * G::BWC + (G::AX - G::CR0) + 2 * lane;
+      if(G::MASK || (s_gcd[3] & 4) == 0)
+      {
+        uint32_t c0[16], c1[4], c2[4], ty[16], tu[4], tv[4];
+        load_test420<R, T>(tst, by, lane, 0, ty, tu, tv);
+        const uint32_t m0 = 0u - 2u * kw0, m1 = 0u - 2u * kw1, m2 = 0u - 2u * kw2;
+        const uint32_t o0 = m0 * (uint32_t)(g0 - mid), o1 = m1 * (uint32_t)(g1 - mid), o2 = m2 * (uint32_t)(g2 - mid);
+        #pragma unroll
+        for(int p = 0; p < 16; p++) { c0[p] = m0 * ty[p] + o0; }
+        #pragma unroll
+        for(int b = 0; b < 4; b++) { c1[b] = m1 * tu[b] + o1; c2[b] = m2 * tv[b] + o2; }
+        // held in registers from here on: recomputed from the test samples at every use they would
+        // cost the search as many multiply-adds again
+        #pragma unroll
+        for(int p = 0; p < 16; p++) { asm volatile("" : "+r"(c0[p])); }
+        #pragma unroll
+        for(int b = 0; b < 4; b++) { asm volatile("" : "+r"(c1[b]), "+r"(c2[b])); }
+        search420<R, T>(luma + (dir ^ 1) * (G::SH * G::LPP) + 4 * by * G::LPP + lane,
+                        chroma + (dir ^ 1) * (G::CH * G::CPP) + 2 * by * G::CPP + lane, c0, c1, c2, idx);
+      }
+      else
+      {
+        uint32_t found[16];
+        search420_literal<R, T>(tst, ref, lofs, cofs, (uint32_t)a.wi[0], (uint32_t)a.wi[1], (uint32_t)a.wi[2], g0, g1, g2, found);
+        #pragma unroll
+        for(int p = 0; p < 16; p++) { idx[p] = found[p]; }
+      }
+      // the test samples are read again: kept through the search they would take 24 registers from it
+      uint32_t ty[16], tu[4], tv[4];
+      int zero = 0;
+      asm volatile("" : "+r"(zero));
+      load_test420<R, T>(tst, by, lane, zero, ty, tu, tv);
+      const uint32_t base = (uint32_t)(lofs * G::ESZ) | ((uint32_t)(cofs * G::ESZ) << 16);
+      if constexpr(G::MASK)
+      {
+        epilogue420_masked<R, T, TM>(a, ref, reinterpret_cast<const TM*>(box + G::OFFM) + (4 * by + R) * G::BWM + G::AXM + 4 * lane, s_off, base, ty, tu,
+                                     tv, idx, dir, xb, yb, g0, g1, g2);
+      }
+      else
+      {
+      const int sel = ((x0 + G::TW > a.W || y0 + G::TH > a.H) ? 4 : 0) | (a.mom[dir].p != nullptr ? 2 : 0) |
+                      ((dir ? a.scp0 : a.scp1) != nullptr ? 1 : 0);
+      switch(sel)
+      {
+      case 0: epilogue420<R, T, false, false, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
+      case 1: epilogue420<R, T, false, false, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
+      case 2: epilogue420<R, T, false, true, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
+      case 4: epilogue420<R, T, true, false, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
+      case 6: epilogue420<R, T, true, true, false>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
+      case 5: epilogue420<R, T, true, false, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;
+      default: epilogue420<R, T, true, true, true>(a, ref, s_off, base, ty, tu, tv, idx, dir, xb, yb, g0, g1, g2); break;   // 3, 7
+      }
+      }
     }
     if(G::STAGES == 1)
     {

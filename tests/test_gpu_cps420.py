@@ -92,3 +92,44 @@ def test_masked_tiles(size, bd, mbd, R, qctx, oracle_lib):
         for planes in ((*f, m), (*[tuple(dev(p, 5) for p in x) for x in f], dev(m, 3)), (*[tuple(dev(p, -p.shape[1] % 16) for p in x) for x in f], dev(m, -W % 16))):
             got, n = calc.compute_masked(*planes, mbd)
             assert n == nnm and {k: got[k] for k in exp} == exp
+
+
+@pytest.mark.parametrize("size", [(262, 34), (520, 66), (392, 50)])
+@pytest.mark.parametrize("bd,mbd,R", [(8, 8, 1), (10, 8, 2), (10, 10, 2), (8, 8, 3), (10, 12, 4), (10, 8, 5)])
+def test_masked_tiles_and_strips_without_pixels(size, bd, mbd, R, qctx, oracle_lib):
+    """Tiles of 128 x 16 and strips of 128 x 4 pixels whose mask is zero are skipped, one kept pixel at any of their
+    corners keeps them: the first, last and inner tiles empty, single pixels, strips past the picture; planes with and
+    without TMA, one pair and batches that mix them."""
+    import torch
+    W, H = size
+    rng = np.random.default_rng(bd * 10 + R + W)
+    top, dt, mdt = (1 << bd) - 1, np.uint8 if bd == 8 else np.uint16, np.uint8 if mbd == 8 else np.uint16
+    f = [tuple(rng.integers(0, top + 1, (H >> s, W >> s)).astype(dt) for s in (0, 1, 1)) for _ in range(2)]
+    def at(*pixels):
+        m = np.zeros((H, W), mdt)
+        for y, x in pixels:
+            m[y, x] = rng.integers(1, 1 << mbd)
+        return m
+    block = np.zeros((H, W), mdt)
+    block[17:30, 130:250] = 3
+    last = np.zeros((H, W), mdt)
+    last[(H - 1) // 16 * 16:, (W - 1) // 128 * 128:] = (1 << mbd) - 1
+    masks = [at((0, 0)), at((H - 1, W - 1)), at((15, 127), (16, 128)), at((3, 128), (4, 127), (H - 1, 0)), block, last]
+    def dev(a, extra):
+        t = torch.zeros(a.shape[0], a.shape[1] + extra, dtype=torch.uint8 if a.dtype == np.uint8 else torch.uint16, device="cuda")
+        t[:, :a.shape[1]] = torch.from_numpy(np.ascontiguousarray(a)).cuda()
+        return t[:, :a.shape[1]]
+    odd = [tuple(dev(p, 5) for p in x) for x in f]
+    even = [tuple(dev(p, -p.shape[1] % 16) for p in x) for x in f]
+    exp = [oracle_lib.compute_pair_masked(oracle.make_params(W, H, bd, 420, search_range=R), *f, m, mbd) for m in masks]
+    want = lambda got, e: {k: got[k] for k in e} == e
+    with qmiv_b200.Calc(qctx, W, H, bd, 420, search_range=R) as calc:
+        for m, (e, n) in zip(masks, exp):
+            for planes, extra in ((odd, 3), (even, -W % 16)):
+                got, nnm = calc.compute_masked(*planes, dev(m, extra), mbd)
+                assert nnm == n and want(got, e)
+    pairs = [dict(frame0=p[0], frame1=p[1], width=W, height=H, bitdepth=bd, search_range=R, metrics="PSNR,WSPSNR,IVPSNR")
+             for _ in masks for p in (odd, even)]
+    with qmiv_b200.Batch(qctx, len(pairs), len(pairs) * W * H) as b:
+        got, nnm = b.compute_masked(pairs, [dev(m, x) for m in masks for x in (3, -W % 16)], [mbd] * len(pairs))
+    assert all(nnm[i] == exp[i // 2][1] and want(got[i], exp[i // 2][0]) for i in range(len(pairs)))
