@@ -46,7 +46,7 @@
 // above every real key and the winners' squared differences are weighted by the test pixels' mask values. A strip of
 // 128 x 4 pixels without a kept one is not searched, a tile without one not staged. Calls of 4096x2048, 10 bits,
 // 8-bit mask, R = 2: full mask 290 us by the fp32-key kernel (one pixel column per thread, tiles staged sample by sample, no
-// copies in flight) -> 162, a disc (31 % of the picture) 214 -> 113, a rectangle of 5 % 184 -> 89; R = 4 452 -> 296,
+// copies in flight) -> 162, a disc (32 % of the picture) 214 -> 113, a rectangle of 5 % 184 -> 89; R = 4 452 -> 296,
 // 270 -> 163, 197 -> 100. Where single 16x16 blocks are strewn over the picture, 20 % of them kept, the strips of
 // 32 x 4 pixels of that kernel left out more: 219 -> 156 at R = 2, 280 -> 287 at R = 4, 367 -> 405 at R = 5. Dealing the
 // kept 4x4 blocks to as few warps as hold them took longer still (424 at R = 4): a tile lasts as long as one warp.

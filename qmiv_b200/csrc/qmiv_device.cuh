@@ -69,8 +69,8 @@ struct Kbns
   // N terms in order where |s| >= |v| is known for each: the larger operand is s, so the compare and the
   // selects go away. The four additions of a term depend on one another, and a lone warp issues in order,
   // so they are written a term apart: the next sum, the difference of the last one, the error of the one
-  // before, the compensation of the one before that. 26 cycles a term written term by term, with or
-  // without the compare, 13 like this (8 is the latency of the sums alone).
+  // before, the compensation of the one before that. WS-PSNR of a 4096x2048 pair whose row errors span more than
+  // ExactSum takes: 63 us a call term by term, 56 like this.
   template <int N>
   __device__ __forceinline__ void add_small(const double (&v)[N])
   {
@@ -164,13 +164,21 @@ struct ExactSum
 
 // Ordered compensated sum of vals[0, n) after `k`, by one thread. all: the terms of the whole chain, for their
 // largest and their signs. While all terms are non-negative the sum never falls, so from the first
-// prefix that reaches the largest term on every addition has |s| >= |v|.
+// prefix that reaches the largest term on every addition has |s| >= |v|. Reached only by chains that ExactSum
+// cannot take.
 __device__ __forceinline__ void chain_sum(Kbns& k, const double* vals, int n, const ExactSum& all)
 {
   int y = 0;
   const double vmax = __hiloint2double((int)(all.top + 1u), 0);
   const bool ordered = (int32_t)all.sign >= 0 && all.top < 0x7fe00000u;   // finite and non-negative
-  for(; y < n && !(ordered && k.s >= vmax); y++) { k.add(vals[y]); }
+  for(; y + 8 <= n && !(ordered && k.s >= vmax); y += 8)     // eight at a time: a call whose largest term comes late took 77 us one by one, 60 so
+  {
+    double v[8];
+    #pragma unroll
+    for(int u = 0; u < 8; u++) { v[u] = vals[y + u]; }
+    #pragma unroll
+    for(int u = 0; u < 8; u++) { k.add(v[u]); }
+  }
   for(; y + 32 <= n; y += 32)
   {
     double v[32];

@@ -79,3 +79,23 @@ def test_tiny_window(qctx, oracle_lib):
     exp = oracle_lib.compute_pair(oracle.make_params(W, H, 8, 420), f0, f1, oracle.SSIM)
     with qmiv_b200.Calc(qctx, W, H, 8, 420) as calc:
         _same(calc.compute(f0, f1, oracle.SSIM), exp, ("ssim",))
+
+
+@pytest.mark.parametrize("H", [14, 16, 18, 254, 1030, 2050])
+@pytest.mark.parametrize("at", [0.0, 0.4, 1.0])
+def test_rows_whose_largest_comes_late(H, at, qctx, oracle_lib):
+    """Rows of one step in one sample and, from the given share of the height on, two rows of full scale: chains
+    that are summed in order, with prefixes of every length before the largest term."""
+    W, bd = 2048, 14
+    a = [np.zeros((H >> s, W >> s), np.uint16) for s in (0, 1, 1)]
+    b = [p.copy() for p in a]
+    for p in b:
+        h = p.shape[0]
+        p[:, 3] = 1
+        y = int(at * (h - 2))
+        p[y:y + 2] = (1 << bd) - 1
+    f0, f1 = tuple(a), tuple(b)
+    mask = oracle.WSPSNR | oracle.IVPSNR
+    exp = oracle_lib.compute_pair(oracle.make_params(W, H, bd, 420, erp=True), f0, f1, mask)
+    with qmiv_b200.Calc(qctx, W, H, bd, 420, erp=True) as calc:
+        _same(calc.compute(f0, f1, mask), exp, ("wspsnr", "ivpsnr", "ivpsnr_r2t", "ivpsnr_t2r"))
