@@ -133,3 +133,24 @@ def test_masked_tiles_and_strips_without_pixels(size, bd, mbd, R, qctx, oracle_l
     with qmiv_b200.Batch(qctx, len(pairs), len(pairs) * W * H) as b:
         got, nnm = b.compute_masked(pairs, [dev(m, x) for m in masks for x in (3, -W % 16)], [mbd] * len(pairs))
     assert all(nnm[i] == exp[i // 2][1] and want(got[i], exp[i // 2][0]) for i in range(len(pairs)))
+
+
+@pytest.mark.parametrize("R", [1, 2, 3, 5])
+def test_work_list_with_and_without_tma(R, qctx, oracle_lib):
+    """One launch over pairs that TMA can and cannot load, in turn: the copies of a tile are issued while the tile
+    before it is searched, whichever way that one was loaded."""
+    import torch
+    W, H, bd = 390, 50, 10
+    f = [synth.make_pair(W, H, bd, seed=20 + i, shift_range=R) for i in range(5)]
+    exp = [oracle_lib.compute_pair(oracle.make_params(W, H, bd, 420, search_range=R), *p, oracle.IVPSNR | oracle.IVSSIM) for p in f]
+    def dev(a, extra):
+        t = torch.zeros(a.shape[0], a.shape[1] + extra, dtype=torch.uint16, device="cuda")
+        t[:, :a.shape[1]] = torch.from_numpy(np.ascontiguousarray(a)).cuda()
+        return t[:, :a.shape[1]]
+    pairs = []
+    for i, p in enumerate(f):
+        a, b = [tuple(dev(x, 3 if i % 2 else -x.shape[1] % 16) for x in fr) for fr in p]
+        pairs.append(dict(frame0=a, frame1=b, width=W, height=H, bitdepth=bd, search_range=R, metrics=["IVPSNR", "IVSSIM"]))
+    with qmiv_b200.Batch(qctx, 40, 40 * W * H) as b:
+        got = b.compute(pairs * 8)
+    assert all({k: got[i][k] for k in exp[i % 5]} == exp[i % 5] for i in range(40))
