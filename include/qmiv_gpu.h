@@ -182,13 +182,13 @@ QMIV_API qmiv_status qmiv_ctx_memory(qmiv_ctx ctx, uint64_t* used_bytes, uint64_
 enum
 {
   QMIV_STAGE_H2D = 0,        /* host frame upload */
-  QMIV_STAGE_PREPASS = 1,    /* per-row SD/SSD */
-  QMIV_STAGE_REDUCE = 2,     /* totals + GCD */
+  QMIV_STAGE_PREPASS = 1,    /* SD, per-row SSD; without a mask also totals and GCD */
+  QMIV_STAGE_REDUCE = 2,     /* mask mode: totals + GCD (0 otherwise) */
   QMIV_STAGE_CPS = 3,        /* corresponding-pixel-shift search, both directions */
   QMIV_STAGE_SSIM_WIN = 4,   /* SSIM windows (+ pyramid downsampling) */
   QMIV_STAGE_SSIM_ROWS = 5,  /* per-row SSIM sums */
-  QMIV_STAGE_FINALIZE = 6,   /* FP64 pooling chains */
-  QMIV_STAGE_D2H = 7,        /* result read-back */
+  QMIV_STAGE_FINALIZE = 6,   /* FP64 pooling chains; one pair: and its result written to the host */
+  QMIV_STAGE_D2H = 7,        /* result read-back by a copy (batches, mask mode, calls without chains) */
   QMIV_NUM_STAGES = 8
 };
 QMIV_API qmiv_status qmiv_ctx_set_profiling(qmiv_ctx ctx, int32_t enable);

@@ -32,12 +32,13 @@
 // A staged luma row keeps its pixel pairs (16 bytes) split by parity of the pair, so the 16-byte loads
 // of a warp (lane stride two pairs) are contiguous; a chroma row's pairs are contiguous as they are.
 //
-// What bounds it: the integer pipes. A warp's tile takes about 2350 instructions at R = 2 with IV-SSIM
-// moments (search 960, epilogue 760, staging 260), of which the multiply-adds keep their pipe busy 60 %
-// of the time at two cycles each and the additions and minima theirs 40 %; issue is at 62 % with 16 warps
-// per SM as with 24. 4096x2048, 10 bits, R = 2, moments: 1239 -> 897 us per 8 pairs (one pair 154 -> 118);
-// without moments and with the compensated pictures stored, 2048x2048: 723 -> 470 us per 8 pairs; 12 bits,
-// 1998x1080 (the literal search before): 262 -> 89 us. Gathering the winners from the staged rows instead,
+// What bounds it: the integer pipes. A warp's tile takes about 2290 instructions at R = 2 with IV-SSIM
+// moments (search 960, epilogue 760, staging 260), of which the multiply-adds keep their pipe busy 63 %
+// of the time at two cycles each and the additions and minima theirs 41 %; issue is at 64 % with 24 warps
+// per SM. 4096x2048, 10 bits, R = 2, moments: 1239 -> 838 us per 8 pairs (one pair 154 -> 111), 897 of it while
+// one kernel served one pair and the work list alike; without moments and with the compensated pictures stored,
+// 2048x2048: 723 -> 447 us per 8 pairs; 12 bits, 1998x1080 (the literal search before): 262 -> 84 us. Against that
+// kernel of 897 and 470 us, gathering the winners from the staged rows instead,
 // which frees the raw boxes for the next tile's copies, measured 918-930 us (bank conflicts); two CTAs
 // with double-buffered boxes measure 883 us with moments but 485 with stored pictures, so the raw boxes
 // are double-buffered only where three CTAs do not fit.
@@ -466,7 +467,9 @@ __device__ __forceinline__ void search420(const uint4* luma, const uint4* chroma
 }
 
 // The same winners by the SSE path's arithmetic taken literally (wrapping int32 errors, first strict
-// minimum in raster order), from the raw boxes of any 16-bit samples.
+// minimum in raster order), from the raw boxes of any 16-bit samples. Bound by its shared-memory loads, three a
+// candidate; a call of 1920x1080, 12 bits, R = 3 / 4 / 5 took 395 / 571 / 1119 us when the literal search ran on
+// float4 tiles, 279 / 410 / 686 like this; 14 bits, R = 2: 247 -> 163.
 template <int R, typename T>
 __device__ __noinline__ void search420_literal(const unsigned char* tst, const unsigned char* ref, int lofs, int cofs,
                                                uint32_t w0, uint32_t w1, uint32_t w2, int g0, int g1, int g2, uint32_t idx[16])

@@ -4,7 +4,7 @@
 //   descriptors   one host-to-device copy of every pair's argument blocks (tensor maps included)
 //   prepass       one launch per sample size, a CTA row per pair, totals and GCD by its last (k_prepass_multi)
 //   CPS           one persistent launch per (R, sample size, tile height) over a work list of the
-//                 tiles of all its pairs                                   (k_cps_multi)
+//                 tiles of all its pairs                     (k_cps420_multi, k_cps_multi)
 //   SSIM          windows of all pairs at scale 0, the smaller scales, their windows, every window row
 //   finalize      one CTA per (pair, pooling chain)                       (k_finalize_multi)
 //   results       one device-to-host copy of all pairs' PairOut

@@ -2,13 +2,13 @@
 //
 // Pipeline of one frame pair (the reference runs the same steps per frame on the CPU,
 // apps/QMIV/src/xAppQMIV.cpp:761-827):
-//   k_prepass   SD(In1-In0), SSD per raw row, max sample (HBM bound, reads both frames once); its last
+//   k_prepass   SD(In1-In0), SSD per raw row, OR of the samples (reads both frames once); its last
 //               CTA: totals, GCD, exactness of the key search path
 //   k_cps       (qmiv_cps.cu, qmiv_cps420.cuh) corresponding-pixel-shift search, both directions in one pass;
 //               per-row SSE into 32-bit lanes, the IV-SSIM sub-block moments of (test, SCP) and,
 //               when IV-MS-SSIM or the caller needs them, the shift-compensated pictures
 //   k_ssim_*    (qmiv_ssim.cu) block SSIM from exact integer moments, FP64 windows, row sums
-//   k_finalize  every order-dependent FP64 pooling chain of the pair (one CTA per chain)
+//   k_finalize  every FP64 pooling chain of the pair (one CTA per chain)
 #include "qmiv_kernels.cuh"
 
 #include <cstdio>

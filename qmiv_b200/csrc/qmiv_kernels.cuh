@@ -25,7 +25,7 @@ cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem
 }
 
 // ---------------------------------------------------------------------------------------------
-// prepass: per raw row of every plane SSD, over the planes SD (In1 - In0), SSD and the largest sample
+// prepass: per raw row of every plane SSD, over the planes SD (In1 - In0), SSD and the OR of the samples
 // per frame; the last CTA forms the totals, the GCD and the path flags
 // ---------------------------------------------------------------------------------------------
 struct PrepassArgs

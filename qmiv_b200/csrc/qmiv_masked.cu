@@ -15,8 +15,9 @@
 //                    k_cps_masked_key is the same search by exact fp32 keys, both directions per
 //                    CTA, four pixels per thread, where the bit depth, weights and GCD range bound
 //                    every error; 4:2:0 pictures take the integer-key search of qmiv_cps420.cuh
-//   k_mask_finalize  the ordered compensated sums (xKBNS.h:36-43) of the ERP row weights and the
-//                    row totals, one CTA per chain (terms staged in shared memory, one thread sums)
+//   k_mask_finalize  the compensated sums (xKBNS.h:36-43) of the ERP row weights and the row totals,
+//                    one CTA per chain, by all its threads (ExactSum), in order by one where the
+//                    terms lie too far apart
 // dB values, exact-component fake values and the picture averages are formed on the host in
 // qmiv_frame_pair_compute_masked with the reference's arithmetic, including its choice of the mask's
 // bit depth for the picture's maximum in PSNR-M (xPSNR.cpp:61) and its direction labels in
